@@ -174,21 +174,31 @@ altob_status fit_from(const double* G, int nmode, int R, const double* lam, cons
     return ALTOB_OK;
 }
 
+// Blocks of the column kernels: eight rows per thread, at most four blocks per SM.
+static int col_grid(u64 I, int R) { return dn_grid(I, (u64)(DN_THREADS / R) * 8); }
+
 template <typename FT>
-altob_status colsum_abs(const FT* U, u64 I, int R, double* acc, cudaStream_t st)
+altob_status colsum_abs_sum(const FT* U, u64 I, int R, double* acc, double* sum, cudaStream_t st)
 {
-    ALTOB_CUDA(cudaMemsetAsync(acc, 0, (size_t)R * sizeof(double), st));
+    if (R > 128) return fail(ALTOB_ERR_UNSUPPORTED, "rank above 128 in the column sums");
     if (I == 0) return ALTOB_OK;
-    k_colsum_abs<FT><<<dn_grid(I * R, DN_THREADS * 16), DN_THREADS, R * sizeof(double), st>>>(U, I, R, acc);
+    k_colsum_abs<FT><<<col_grid(I, R), DN_THREADS, (R + 1) * sizeof(double), st>>>(U, I, R, acc, sum);
     ALTOB_LAUNCH_CHECK();
     return ALTOB_OK;
 }
 
 template <typename FT>
-altob_status div_cols(FT* U, u64 I, int R, const double* d, cudaStream_t st)
+altob_status colsum_abs(const FT* U, u64 I, int R, double* acc, cudaStream_t st)
 {
-    if (I == 0) return ALTOB_OK;
-    k_scale_cols<FT><<<dn_grid(I * R, DN_THREADS * 8), DN_THREADS, 0, st>>>(U, I, R, d, 1);
+    ALTOB_CUDA(cudaMemsetAsync(acc, 0, (size_t)R * sizeof(double), st));
+    return colsum_abs_sum<FT>(U, I, R, acc, nullptr, st);
+}
+
+template <typename FT>
+altob_status div_cols(FT* U, u64 I, int R, const double* d, double* lam, bool set_lam, cudaStream_t st)
+{
+    if (R > 128) return fail(ALTOB_ERR_UNSUPPORTED, "rank above 128 in the column scaling");
+    k_scale_cols<FT><<<col_grid(I, R), DN_THREADS, 0, st>>>(U, I, R, d, 1, lam, set_lam);
     ALTOB_LAUNCH_CHECK();
     return ALTOB_OK;
 }
@@ -196,32 +206,16 @@ altob_status div_cols(FT* U, u64 I, int R, const double* d, cudaStream_t st)
 template <typename FT>
 altob_status mul_cols(FT* U, u64 I, int R, const double* d, cudaStream_t st)
 {
+    if (R > 128) return fail(ALTOB_ERR_UNSUPPORTED, "rank above 128 in the column scaling");
     if (I == 0) return ALTOB_OK;
-    k_scale_cols<FT><<<dn_grid(I * R, DN_THREADS * 8), DN_THREADS, 0, st>>>(U, I, R, d, 0);
-    ALTOB_LAUNCH_CHECK();
-    return ALTOB_OK;
-}
-
-template <typename FT>
-altob_status sum_all(const FT* U, u64 n, double* acc, cudaStream_t st)
-{
-    ALTOB_CUDA(cudaMemsetAsync(acc, 0, sizeof(double), st));
-    if (n == 0) return ALTOB_OK;
-    k_sum_all<FT><<<dn_grid(n, DN_THREADS * 16), DN_THREADS, 0, st>>>(U, n, acc);
-    ALTOB_LAUNCH_CHECK();
-    return ALTOB_OK;
-}
-
-altob_status vec_mul(double* lam, const double* d, int R, cudaStream_t st)
-{
-    k_vec<<<1, 128, 0, st>>>(lam, d, R, 0.0, 0);
+    k_scale_cols<FT><<<col_grid(I, R), DN_THREADS, 0, st>>>(U, I, R, d, 0, nullptr, 0);
     ALTOB_LAUNCH_CHECK();
     return ALTOB_OK;
 }
 
 altob_status vec_fill(double* v, int R, double x, cudaStream_t st)
 {
-    k_vec<<<1, 128, 0, st>>>(v, nullptr, R, x, 1);
+    k_vec<<<1, 128, 0, st>>>(v, R, x);
     ALTOB_LAUNCH_CHECK();
     return ALTOB_OK;
 }
@@ -262,9 +256,9 @@ altob_status value_sumsq(const altob_tensor* t, double* acc, cudaStream_t st)
                                          cudaStream_t);                                                      \
     template altob_status normalize_cols<FT>(FT*, u64, int, const double*, cudaStream_t);                    \
     template altob_status colsum_abs<FT>(const FT*, u64, int, double*, cudaStream_t);                        \
-    template altob_status div_cols<FT>(FT*, u64, int, const double*, cudaStream_t);                          \
+    template altob_status colsum_abs_sum<FT>(const FT*, u64, int, double*, double*, cudaStream_t);           \
+    template altob_status div_cols<FT>(FT*, u64, int, const double*, double*, bool, cudaStream_t);           \
     template altob_status mul_cols<FT>(FT*, u64, int, const double*, cudaStream_t);                          \
-    template altob_status sum_all<FT>(const FT*, u64, double*, cudaStream_t);                                \
     template altob_status vec_to<FT>(FT*, const double*, int, cudaStream_t);                                 \
     template altob_status vec_from<FT>(double*, const FT*, int, cudaStream_t);
 

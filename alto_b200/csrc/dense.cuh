@@ -46,13 +46,14 @@ altob_status fit_from(const double* G, int nmode, int R, const double* lam, cons
                       double* fit, cudaStream_t st);
 template <typename FT>
 altob_status colsum_abs(const FT* U, u64 I, int R, double* acc, cudaStream_t st);
+// The same into zeroed accumulators, with the plain sum of every element.
 template <typename FT>
-altob_status div_cols(FT* U, u64 I, int R, const double* d, cudaStream_t st);
+altob_status colsum_abs_sum(const FT* U, u64 I, int R, double* acc, double* sum, cudaStream_t st);
+// U /= d column-wise; lam *= d, or lam = d with set_lam (lam known to be 1).
+template <typename FT>
+altob_status div_cols(FT* U, u64 I, int R, const double* d, double* lam, bool set_lam, cudaStream_t st);
 template <typename FT>
 altob_status mul_cols(FT* U, u64 I, int R, const double* d, cudaStream_t st);
-template <typename FT>
-altob_status sum_all(const FT* U, u64 n, double* acc, cudaStream_t st);
-altob_status vec_mul(double* lam, const double* d, int R, cudaStream_t st);
 altob_status vec_fill(double* v, int R, double x, cudaStream_t st);
 template <typename FT>
 altob_status vec_to(FT* dst, const double* src, int R, cudaStream_t st);

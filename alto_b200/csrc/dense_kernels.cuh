@@ -824,42 +824,63 @@ static __global__ void k_fit(const double* __restrict__ G, int nmode, int R, con
     fit_body(G, nmode, R, lam, inner, normAT, fit);
 }
 
+// Column kernels over an I x R matrix: a thread stays on one column (the
+// threads of a block past the last whole row idle), so the element loop has
+// no division by R and a column sum is a register until the block's end.
+
+// acc[r] += sum_i |U[i, r]|; sum (if given) += sum of all elements.
 template <typename FT>
-static __global__ void k_colsum_abs(const FT* __restrict__ U, u64 I, int R, double* __restrict__ acc)
+static __global__ void __launch_bounds__(DN_THREADS) k_colsum_abs(const FT* __restrict__ U, u64 I, int R,
+                                                                  double* __restrict__ acc, double* __restrict__ sum)
 {
-    extern __shared__ double cs_[];
-    for (int r = threadIdx.x; r < R; r += blockDim.x) cs_[r] = 0.0;
+    extern __shared__ double cs_[];  // R column sums, then the plain sum
+    for (int r = threadIdx.x; r <= R; r += blockDim.x) cs_[r] = 0.0;
     __syncthreads();
-    const u64 n = I * (u64)R;
-    for (u64 e = (u64)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (u64)gridDim.x * blockDim.x)
-        atomicAdd(&cs_[e % R], fabs((double)U[e]));
+    const int rpb = DN_THREADS / R;  // rows per block step (R <= 128)
+    const int row = threadIdx.x / R, col = threadIdx.x - row * R;
+    double a = 0.0, t = 0.0;
+    if (row < rpb) {
+        const u64 step = (u64)gridDim.x * rpb;
+#pragma unroll 4
+        for (u64 i = (u64)blockIdx.x * rpb + row; i < I; i += step) {
+            const double x = (double)U[i * R + col];
+            a += fabs(x);
+            t += x;
+        }
+        atomicAdd(&cs_[col], a);
+    }
+    if (sum) {
+        for (int o = 16; o; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        if ((threadIdx.x & 31) == 0) atomicAdd(&cs_[R], t);
+    }
     __syncthreads();
     for (int r = threadIdx.x; r < R; r += blockDim.x) atomicAdd(&acc[r], cs_[r]);
+    if (sum && threadIdx.x == 0) atomicAdd(sum, cs_[R]);
 }
 
+// U[i, r] *= d[r] (or /= d[r]); lam (if given) *= d, or = d with set_lam.
 template <typename FT>
-static __global__ void k_scale_cols(FT* __restrict__ U, u64 I, int R, const double* __restrict__ d, int divide)
+static __global__ void __launch_bounds__(DN_THREADS) k_scale_cols(FT* __restrict__ U, u64 I, int R,
+                                                                  const double* __restrict__ d, int divide,
+                                                                  double* __restrict__ lam, int set_lam)
 {
-    const u64 n = I * (u64)R;
-    for (u64 e = (u64)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (u64)gridDim.x * blockDim.x) {
-        const double v = (double)U[e];
-        U[e] = (FT)(divide ? v / d[e % R] : v * d[e % R]);
+    const int rpb = DN_THREADS / R;
+    const int row = threadIdx.x / R, col = threadIdx.x - row * R;
+    if (lam && blockIdx.x == 0)
+        for (int r = threadIdx.x; r < R; r += blockDim.x) lam[r] = set_lam ? d[r] : lam[r] * d[r];
+    if (row >= rpb) return;
+    const double dc = d[col];
+    const u64 step = (u64)gridDim.x * rpb;
+#pragma unroll 4
+    for (u64 i = (u64)blockIdx.x * rpb + row; i < I; i += step) {
+        const double v = (double)U[i * R + col];
+        U[i * R + col] = (FT)(divide ? v / dc : v * dc);
     }
 }
 
-template <typename FT>
-static __global__ void k_sum_all(const FT* __restrict__ U, u64 n, double* __restrict__ acc)
+static __global__ void k_vec(double* v, int R, double x)
 {
-    double s = 0.0;
-    for (u64 e = (u64)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (u64)gridDim.x * blockDim.x)
-        s += (double)U[e];
-    for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if ((threadIdx.x & 31) == 0) atomicAdd(acc, s);
-}
-
-static __global__ void k_vec(double* lam, const double* d, int R, double x, int op)
-{
-    for (int r = threadIdx.x; r < R; r += blockDim.x) lam[r] = op == 0 ? lam[r] * d[r] : x;
+    for (int r = threadIdx.x; r < R; r += blockDim.x) v[r] = x;
 }
 
 template <typename A, typename B>
