@@ -494,8 +494,8 @@ struct BatchImpl : BatchBase {
     }
 
     // Uploads per-mode tables for (tensor, slots) members; returns counts.
-    // planned: 1 = the members whose mode has a tile plan, 0 = the others
-    // (a class whose kernel shape has no planned form keeps every member in
+    // planned: 1 = the members whose mode has a tile plan or is read through
+    // oidx (in target order already), 0 = the others (a class whose kernel shape has no planned form keeps every member in
     // the grouped tables)
     altob_status upload_tables(const std::vector<std::pair<int, int>>& mem, int planned, bool plan_shape,
                                TiledArgs<FT>** d_args, u64** d_prefix, int** d_bid, u64* total_tiles, int* count,
@@ -509,7 +509,8 @@ struct BatchImpl : BatchBase {
             for (const auto& m : mem) {
                 if (ts[m.first]->nmode <= j) continue;
                 TiledArgs<FT> a = make_args(m.first, j, m.second, plan_shape, st);
-                if ((a.plan != nullptr) != (planned != 0)) continue;
+                const bool in_plan = a.plan != nullptr || (plan_shape && a.perm != nullptr);
+                if (in_plan != (planned != 0)) continue;
                 args.push_back(a);
                 prefix.push_back(tiles);
                 bid.push_back(m.first);
@@ -549,7 +550,7 @@ struct BatchImpl : BatchBase {
         pp.free_args();
         if (!plan_shape(nm, vec, ch)) return ALTOB_OK;
         ALTOB_TRY(upload_tables(mem, 1, true, pp.d_args, pp.d_prefix, pp.d_bid, pp.total_tiles, pp.count, st));
-        pp.smem = planned_batch_smem(nm, sizeof(FT));
+        pp.smem = planned_batch_smem(nm, sizeof(FT), lpn);
         BatchTiles<FT> bt;
         memset(&bt, 0, sizeof(bt));
         int bps = 0;

@@ -67,22 +67,7 @@ altob_status tensor_scratch(altob_tensor* t, size_t bytes, void** out)
     return ALTOB_OK;
 }
 
-altob_status tensor_hotbuf(altob_tensor* t, size_t bytes, void** out)
-{
-    if (bytes > t->hotbuf_bytes) {
-        if (t->hotbuf) {
-            dfree(t->hotbuf);
-            t->hotbuf = nullptr;
-            t->hotbuf_bytes = 0;
-        }
-        ALTOB_TRY(dmalloc(&t->hotbuf, bytes));
-        t->hotbuf_bytes = bytes;
-    }
-    *out = t->hotbuf;
-    return ALTOB_OK;
-}
-
-static bool capturing(cudaStream_t st)
+bool stream_capturing(cudaStream_t st)
 {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(st, &cs) != cudaSuccess) {
@@ -92,16 +77,44 @@ static bool capturing(cudaStream_t st)
     return cs != cudaStreamCaptureStatusNone;
 }
 
+// Buffers that outlive the call are never grown while st is being captured:
+// the allocation would belong to the graph.
+static altob_status grow_buf(void** buf, size_t* have, size_t bytes, void** out, cudaStream_t st)
+{
+    if (bytes > *have) {
+        if (stream_capturing(st)) return fail(ALTOB_ERR_NOMEM, "a handle's buffer cannot grow during stream capture");
+        if (*buf) {
+            dfree(*buf);
+            *buf = nullptr;
+            *have = 0;
+        }
+        ALTOB_TRY(dmalloc(buf, bytes));
+        *have = bytes;
+    }
+    *out = *buf;
+    return ALTOB_OK;
+}
+
+altob_status tensor_hotbuf(altob_tensor* t, size_t bytes, void** out, cudaStream_t st)
+{
+    return grow_buf(&t->hotbuf, &t->hotbuf_bytes, bytes, out, st);
+}
+
+altob_status tensor_padbuf(altob_tensor* t, size_t bytes, void** out, cudaStream_t st)
+{
+    return grow_buf(&t->padbuf, &t->padbuf_bytes, bytes, out, st);
+}
+
 altob_status tensor_enter(altob_tensor* t, cudaStream_t st)
 {
-    if (!t->use_ev || t->use_stream == st || capturing(st)) return ALTOB_OK;
+    if (!t->use_ev || t->use_stream == st || stream_capturing(st)) return ALTOB_OK;
     ALTOB_CUDA(cudaStreamWaitEvent(st, t->use_ev, 0));
     return ALTOB_OK;
 }
 
 altob_status tensor_leave(altob_tensor* t, cudaStream_t st)
 {
-    if (capturing(st)) return ALTOB_OK;
+    if (stream_capturing(st)) return ALTOB_OK;
     if (!t->use_ev) ALTOB_CUDA(cudaEventCreateWithFlags(&t->use_ev, cudaEventDisableTiming));
     ALTOB_CUDA(cudaEventRecord(t->use_ev, st));
     t->use_stream = st;
@@ -1161,6 +1174,7 @@ altob_status altob_destroy(altob_tensor* t)
     for (int n = 0; n < ALTOB_MAX_MODES; ++n) dfree(t->d_plan[n]);
     dfree(t->scratch);
     dfree(t->hotbuf);
+    dfree(t->padbuf);
     dfree(t->d_tma_err);
     if (t->h_tma_err) {
         cudaStreamSynchronize(0);  // the flag's last copy was ordered before the frees above

@@ -211,6 +211,9 @@ struct altob_tensor {
     // per-CTA hot-row accumulators of the grouped kernel (grown on demand)
     void* hotbuf = nullptr;
     size_t hotbuf_bytes = 0;
+    // padded factor copies of ranks without vector rows (grown on demand)
+    void* padbuf = nullptr;
+    size_t padbuf_bytes = 0;
     // tile plans of the planned MTTKRP kernel, one per mode (built on first use)
     uint16_t* d_plan[ALTOB_MAX_MODES] = {nullptr};
     // the TMA-staged kernel's wait-limit flag: on the device, and a pinned
@@ -259,7 +262,10 @@ void dfree(void* p);
 // Per-tensor scratch: returns a device buffer of at least `bytes`, reused
 // across calls on the same handle.
 altob_status tensor_scratch(altob_tensor* t, size_t bytes, void** out);
-altob_status tensor_hotbuf(altob_tensor* t, size_t bytes, void** out);
+// Whether work issued on st goes into a graph under capture.
+bool stream_capturing(cudaStream_t st);
+altob_status tensor_hotbuf(altob_tensor* t, size_t bytes, void** out, cudaStream_t st);
+altob_status tensor_padbuf(altob_tensor* t, size_t bytes, void** out, cudaStream_t st);
 
 // Stream ordering of a handle's shared state (scratch, hot-row buffers, tile
 // plans): tensor_enter makes stream st wait for the last call that used the

@@ -79,17 +79,22 @@ altob_status plan_tiled(const altob_tensor* t, u64 R, size_t fsz, bool aligned, 
 }
 
 // Per-CTA hot-row accumulator regions for a launch of `grid` CTAs (none when
-// the kernel has no hot-row slots).
+// the kernel has no hot-row slots; during stream capture a handle without a
+// large enough region runs without slots).
 template <typename FT>
 static altob_status set_hot_acc(altob_tensor* t, TiledArgs<FT>& a, unsigned grid, cudaStream_t st)
 {
-    (void)st;
     a.hot_acc = nullptr;
-    if (!a.hot) return ALTOB_OK;
+    const int slots = a.whole ? a.whole : a.hot;
+    if (!slots) return ALTOB_OK;
     void* p = nullptr;
-    ALTOB_TRY(tensor_hotbuf(t, (size_t)grid * a.hot * a.R * sizeof(FT), &p));
+    const altob_status s = tensor_hotbuf(t, (size_t)grid * slots * a.R * sizeof(FT), &p, st);
+    if (s != ALTOB_OK && stream_capturing(st)) {
+        a.hot = a.whole = 0;
+        return ALTOB_OK;
+    }
     a.hot_acc = (FT*)p;
-    return ALTOB_OK;
+    return s;
 }
 
 // Tile plan of `mode` (k_tile_plan), built on the first call that needs it.
@@ -98,10 +103,11 @@ static altob_status set_hot_acc(altob_tensor* t, TiledArgs<FT>& a, unsigned grid
 static bool ensure_plan(altob_tensor* t, int mode, cudaStream_t st)
 {
     if (t->d_plan[mode]) return true;
+    if (stream_capturing(st)) return false;  // the plan outlives the graph
     void* p = nullptr;
     if (dmalloc(&p, (size_t)t->nnz * sizeof(uint16_t)) != ALTOB_OK) return false;
     const u64 ntiles = (t->nnz + PT_TILE - 1) / PT_TILE;
-    k_tile_plan<PT_TILE><<<(unsigned)ntiles, PT_TILE / 2, 0, st>>>(key_src(t), t->fld, t->nnz, mode, (u16*)p);
+    k_tile_plan<PT_TILE><<<(unsigned)ntiles, PT_TILE / TP_IPT, 0, st>>>(key_src(t), t->fld, t->nnz, mode, (u16*)p);
     if (cudaGetLastError() != cudaSuccess) {
         dfree(p);
         return false;
@@ -211,6 +217,109 @@ static altob_status run_tma(altob_tensor* t, TiledArgs<float>& a, u64 R, cudaStr
     return ALTOB_OK;
 }
 
+// Largest output (bytes) that every CTA of the planned kernel keeps a copy of.
+constexpr u64 WHOLE_BYTES = 64 * 1024;
+
+// ------------------------------------------------ ranks without vector rows
+//
+// A rank that is no multiple of a 16-byte vector, or a factor that does not
+// start on one, cannot be gathered in 16-byte pieces.  Such calls run on
+// copies of the factors with the rows padded to whole vectors (zeros past the
+// rank change no product, dot product or sum) and the result is added back:
+// three streaming passes over the factors instead of one 4- or 8-byte load
+// per lane and nonzero.
+
+constexpr int PAD_MATRICES = ALTOB_MAX_MODES + 1;  // every factor (Phi reads the target's too) and the output
+
+struct PadArgs {
+    const void* src[PAD_MATRICES];
+    void* dst[PAD_MATRICES];
+    u64 rows[PAD_MATRICES];
+    int R, Rp;
+};
+
+// dst[m] (rows x Rp) = src[m] (rows x R), zeros past the rank or, without a
+// source, everywhere; matrix m = blockIdx.y.
+template <typename FT>
+__global__ void __launch_bounds__(256) k_pad_rows(PadArgs a)
+{
+    const int m = blockIdx.y;
+    const FT* __restrict__ src = reinterpret_cast<const FT*>(a.src[m]);
+    FT* __restrict__ dst = reinterpret_cast<FT*>(a.dst[m]);
+    if (!dst) return;
+    const int rpb = 256 / a.Rp, row = threadIdx.x / a.Rp, col = threadIdx.x - row * a.Rp;
+    if (row >= rpb) return;
+    const u64 step = (u64)gridDim.x * rpb;
+#pragma unroll 4
+    for (u64 i = (u64)blockIdx.x * rpb + row; i < a.rows[m]; i += step)
+        dst[i * a.Rp + col] = src && col < a.R ? src[i * a.R + col] : FT(0);
+}
+
+// out (rows x R) += src (rows x Rp).
+template <typename FT>
+__global__ void __launch_bounds__(256) k_unpad_add(FT* __restrict__ out, const FT* __restrict__ src, u64 rows, int R,
+                                                   int Rp)
+{
+    const int rpb = 256 / R, row = threadIdx.x / R, col = threadIdx.x - row * R;
+    if (row >= rpb) return;
+    const u64 step = (u64)gridDim.x * rpb;
+#pragma unroll 4
+    for (u64 i = (u64)blockIdx.x * rpb + row; i < rows; i += step) out[i * R + col] += src[i * Rp + col];
+}
+
+static unsigned pad_grid(u64 rows, int R)
+{
+    return (unsigned)std::max<u64>(1, std::min<u64>((rows * (u64)R + 2047) / 2048, (u64)num_sms() * 8));
+}
+
+template <typename FT, typename VT>
+static altob_status run_tiled_vt(altob_tensor* t, int mode, void* const* dU, void* dout, u64 R, bool phi,
+                                 double eps, const u32* perm, bool cache, cudaStream_t st);
+
+// MTTKRP / Phi on padded copies of the factors; *ran = false when the copies
+// cannot be allocated (the caller then runs the scalar-row kernel).
+template <typename FT, typename VT>
+static altob_status run_padded(altob_tensor* t, int mode, void* const* dU, void* dout, u64 R, bool phi, double eps,
+                               const u32* perm, cudaStream_t st, bool* ran)
+{
+    constexpr u64 V = 16 / sizeof(FT);
+    const u64 Rp = (R + V - 1) / V * V;
+    *ran = false;
+    u64 elems = 0, most = 0, off[ALTOB_MAX_MODES], out_off = 0;
+    for (int m = 0; m < t->nmode; ++m) {
+        off[m] = elems;
+        if (m != mode || phi) elems += t->dims[m] * Rp;
+        most = std::max(most, t->dims[m]);
+    }
+    out_off = elems;
+    elems += t->dims[mode] * Rp;
+    void* base = nullptr;
+    if (tensor_padbuf(t, elems * sizeof(FT), &base, st) != ALTOB_OK) return ALTOB_OK;
+    PadArgs pa;
+    memset(&pa, 0, sizeof(pa));
+    void* pU[ALTOB_MAX_MODES] = {nullptr};
+    FT* po = (FT*)base + out_off;
+    int n = 0;
+    for (int m = 0; m < t->nmode; ++m) {
+        pU[m] = m != mode || phi ? (void*)((FT*)base + off[m]) : (void*)po;
+        if (m == mode && !phi) continue;
+        pa.src[n] = dU[m];
+        pa.dst[n] = pU[m];
+        pa.rows[n++] = t->dims[m];
+    }
+    pa.dst[n] = po;
+    pa.rows[n++] = t->dims[mode];
+    pa.R = (int)R;
+    pa.Rp = (int)Rp;
+    k_pad_rows<FT><<<dim3(pad_grid(most, (int)Rp), n), 256, 0, st>>>(pa);
+    ALTOB_LAUNCH_CHECK();
+    ALTOB_TRY((run_tiled_vt<FT, VT>(t, mode, pU, po, Rp, phi, eps, perm, true, st)));
+    k_unpad_add<FT><<<pad_grid(t->dims[mode], (int)R), 256, 0, st>>>((FT*)dout, po, t->dims[mode], (int)R, (int)Rp);
+    ALTOB_LAUNCH_CHECK();
+    *ran = true;
+    return ALTOB_OK;
+}
+
 template <typename FT, typename VT>
 static altob_status run_tiled_vt(altob_tensor* t, int mode, void* const* dU, void* dout, u64 R, bool phi,
                                  double eps, const u32* perm, bool cache, cudaStream_t st)
@@ -219,10 +328,21 @@ static altob_status run_tiled_vt(altob_tensor* t, int mode, void* const* dU, voi
     for (int m = 0; m < t->nmode; ++m) aligned = aligned && ptr_aligned16(dU[m]);
     TiledPlan pl;
     ALTOB_TRY(plan_tiled(t, R, sizeof(FT), aligned, cache, &pl));
-    // MTTKRP of a static order 3-5 in ALTO order with one vector chunk per
-    // lane: the planned kernel (ALTOB_PLAN=0 keeps the grouped kernel)
-    const bool planned = pl.grouped && !phi && !perm && cache && t->nmode >= 3 && t->nmode <= 5 && pl.vec > 1 &&
-                         pl.ch == 1 && t->nnz < (1ull << 32) && env_int("ALTOB_PLAN", 1) && ensure_plan(t, mode, st);
+    // The planned kernel takes static orders 3-5 in ALTO order (or in target
+    // order through oidx) on vector rows; ALTOB_PLAN=0 keeps the grouped one.
+    const bool plannable = pl.grouped && (cache || perm) && t->nmode >= 3 && t->nmode <= 5 && t->nnz < (1ull << 32) &&
+                           env_int("ALTOB_PLAN", 1);
+    if (plannable && pl.vec == 1) {
+        u64 rows = 0;
+        for (int m = 0; m < t->nmode; ++m) rows += t->dims[m];
+        if (t->nnz >= rows) {
+            bool ran = false;
+            ALTOB_TRY((run_padded<FT, VT>(t, mode, dU, dout, R, phi, eps, perm, st, &ran)));
+            if (ran) return ALTOB_OK;
+        }
+    }
+    const bool planned = plannable && pl.vec > 1 && (pl.ch == 1 || (pl.ch == 2 && pl.lpn == 32 && sizeof(FT) == 8)) &&
+                         (perm || ensure_plan(t, mode, st));
     TiledArgs<FT> a;
     memset(&a, 0, sizeof(a));
     a.key = key_src(t);
@@ -256,17 +376,38 @@ static altob_status run_tiled_vt(altob_tensor* t, int mode, void* const* dU, voi
         // Zipf tensor) at the same FP32 error (1.0-1.7e-6 against FP64); below
         // 8 the lookups cost more than the atomics they save (2: 2.61 ms)
         a.hot_minrun = 16;
+        a.hot = env_int("ALTOB_HOT_ROWS", 1) ? hot_slots((int)R, sizeof(FT)) : 0;
         a.tile = PT_TILE;
         a.ntiles = (t->nnz + PT_TILE - 1) / PT_TILE;
         a.hslots = 0;
         if constexpr (sizeof(FT) == 4 && std::is_same<VT, float>::value) {
-            if (tma_eligible(t, R, true)) return run_tma(t, a, R, st);
+            if (!phi && !perm && tma_eligible(t, R, true)) return run_tma(t, a, R, st);
         }
-        const int nbuf = t->nmode == 3 ? planned_nbuf<FT, 3>() : 2;
+        const int nbuf = t->nmode == 3 ? planned_nbuf<FT, 3>() : planned_nbuf<FT, 4>();
         c.smem = planned_smem(t->nmode, sizeof(FT), a.hot, c.lpn, PT_TILE, nbuf);
         ALTOB_TRY((launch_planned<FT, VT>(a, c, st, &bps)));
         if (bps < 1) return fail(ALTOB_ERR_UNSUPPORTED, "planned MTTKRP kernel does not fit on an SM");
-        c.grid = dim3((unsigned)std::max<u64>(1, std::min<u64>(a.ntiles, (u64)bps * num_sms())));
+        // a tensor with fewer tiles than resident CTAs shares each tile among
+        // 2^split_shift CTAs (at least two records per lane group each):
+        // 40,000 nonzeros, order 3, rank 16, FP64: 8.0 -> 6.2 us a mode;
+        // 150,001 nonzeros, order 5, rank 64, FP32: 25 -> 15
+        const u64 cap = (u64)bps * num_sms();
+        const int ipg = planned_ipg(PT_TILE, c.lpn);
+        while ((a.ntiles << (a.split_shift + 1)) <= cap && (ipg >> (a.split_shift + 1)) >= 2) ++a.split_shift;
+        const u64 items = a.ntiles << a.split_shift;
+        c.grid = dim3((unsigned)std::max<u64>(1, std::min<u64>(items, cap)));
+        const u64 per_cta = a.ntiles / c.grid.x;
+        // one item per CTA: a hot-row table would pass every run on unchanged;
+        // in FP64, where it only saves contended atomics, it repays clearing
+        // and adding it up from about four tiles per CTA on
+        if (items <= cap || (sizeof(FT) == 8 && per_cta < 4)) a.hot = 0;
+        // an output of at most WHOLE_BYTES is kept whole by every CTA that
+        // takes enough tiles to repay clearing the copy and adding it up
+        if (!perm && t->dims[mode] * R * sizeof(FT) <= WHOLE_BYTES && t->dims[mode] <= 128 * per_cta && per_cta >= 2 &&
+            env_int("ALTOB_HOT_ROWS", 1)) {
+            a.hot = 0;
+            a.whole = (int)t->dims[mode];
+        }
         ALTOB_TRY(set_hot_acc(t, a, c.grid.x, st));
         return launch_planned<FT, VT>(a, c, st, nullptr);
     }

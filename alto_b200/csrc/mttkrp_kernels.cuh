@@ -162,6 +162,8 @@ struct TiledArgs {
     FT* hot_acc;   // gridDim.x x hot x R accumulators, one private region per CTA
     const uint16_t* plan;  // tile plan of the target mode (planned kernel only)
     int hot_minrun;        // shortest run through the hot-row table (0: GT_HOT_MINRUN)
+    int whole;             // planned kernel: output rows every CTA keeps a copy of (0: none; then hot = 0)
+    int split_shift;       // planned kernel: 2^split_shift CTAs share a tile
 };
 
 // Dynamic shared-memory bytes of k_tiled.
@@ -510,14 +512,18 @@ inline size_t grouped_smem(int hslots, int mm, size_t fsz, int hot = 0, int R = 
 // contention) and reach the output once per CTA instead of once per tile.
 // Rows that many tiles touch (the head of a skewed mode) then take a few
 // hundred FP32 additions instead of one per tile, which keeps their rounding
-// error near the per-tile level.  16 KB per CTA; FP32 only.
-inline int grouped_hot_slots(int R, size_t fsz)
+// error near the per-tile level.  16 KB per CTA.  The grouped kernel uses it
+// for FP32 only; the planned one also for FP64, where it takes the contended
+// atomics off the head rows (28.8M nonzeros of a Zipf tensor, rank 32: 2.42
+// -> 1.93 ms a mode).
+inline int hot_slots(int R, size_t fsz)
 {
-    if (fsz != 4 || R < 1) return 0;
+    if (R < 1) return 0;
     int h = 1;
     while (h * 2 <= 256 && (size_t)(h * 2) * R * fsz <= 16384) h *= 2;
     return h >= 16 ? h : 0;
 }
+inline int grouped_hot_slots(int R, size_t fsz) { return fsz == 4 ? hot_slots(R, fsz) : 0; }
 
 // Slot of run-ordered record p: one padding record after every 32, so the
 // stretches that the lane groups of a warp read at the same time start in

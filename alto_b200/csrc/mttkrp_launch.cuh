@@ -24,7 +24,7 @@ altob_status launch_tiled(const TiledArgs<FT>& a, const TiledCfg& c, cudaStream_
 template <typename FT, typename VT>
 altob_status launch_atomic_cr(const CrArgsK<FT>& a, cudaStream_t st);
 
-// Planned MTTKRP (static order 3-5, one VEC-wide chunk per lane, a.plan set).
+// Planned MTTKRP or Phi (c.phi): static order 3-5, vector rows, a.plan or a.perm set.
 template <typename FT, typename VT>
 altob_status launch_planned(const TiledArgs<FT>& a, const TiledCfg& c, cudaStream_t st, int* bps);
 
@@ -109,30 +109,40 @@ altob_status launch_shape(const TiledArgs<FT>& a, const TiledCfg& c, cudaStream_
     return fail(ALTOB_ERR_UNSUPPORTED, "lanes per nonzero");
 }
 
-template <typename FT, typename VT, int NM, int LPN, int V>
+template <typename FT, typename VT, int NM, int LPN, int V, int CH, bool PHI>
 altob_status launch_planned_one(const TiledArgs<FT>& a, const TiledCfg& c, cudaStream_t st, int* bps)
 {
-    static std::atomic<size_t> configured{0};
-    constexpr int mb = planned_min_blocks<FT, NM, LPN>();
-    if constexpr (mb > 0)
-        return launch_kernel(k_planned_mb<FT, VT, NM, LPN, V, mb, PT_TILE, planned_nbuf<FT, NM>()>, configured, &a, c, st,
-                             bps);
-    else
-        return launch_kernel(k_planned<FT, VT, NM, LPN, V>, configured, &a, c, st, bps);
+    static std::atomic<size_t> configured{0}, configured_perm{0}, configured_whole{0};
+    constexpr int mb = planned_min_blocks<FT, NM, LPN, CH, PHI>(), nb = planned_nbuf<FT, NM>();
+    if constexpr (!PHI) {  // Phi reads in ALTO order only
+        if (a.perm)
+            return launch_kernel(k_planned<FT, VT, NM, LPN, V, CH, PHI, true, false, mb, PT_TILE, nb>, configured_perm, &a,
+                                 c, st, bps);
+    }
+    if (a.whole)
+        return launch_kernel(k_planned<FT, VT, NM, LPN, V, CH, PHI, false, true, mb, PT_TILE, nb>, configured_whole, &a, c,
+                             st, bps);
+    return launch_kernel(k_planned<FT, VT, NM, LPN, V, CH, PHI, false, false, mb, PT_TILE, nb>, configured, &a, c, st,
+                         bps);
 }
 
-template <typename FT, typename VT, int NM>
+template <typename FT, typename VT, int NM, bool PHI>
 altob_status launch_planned_shape(const TiledArgs<FT>& a, const TiledCfg& c, cudaStream_t st, int* bps)
 {
     constexpr int V = 16 / sizeof(FT);
-    if (c.ch != 1) return fail(ALTOB_ERR_UNSUPPORTED, "planned kernel shape");
     if (c.vec != V) return fail(ALTOB_ERR_UNSUPPORTED, "planned kernel shape");
+    if (c.ch == 2) {  // FP64 ranks above 64
+        if constexpr (sizeof(FT) == 8) {
+            if (c.lpn == 32) return launch_planned_one<FT, VT, NM, 32, V, 2, PHI>(a, c, st, bps);
+        }
+        return fail(ALTOB_ERR_UNSUPPORTED, "planned kernel shape");
+    }
     switch (c.lpn) {
-    case 2: return launch_planned_one<FT, VT, NM, 2, V>(a, c, st, bps);
-    case 4: return launch_planned_one<FT, VT, NM, 4, V>(a, c, st, bps);
-    case 8: return launch_planned_one<FT, VT, NM, 8, V>(a, c, st, bps);
-    case 16: return launch_planned_one<FT, VT, NM, 16, V>(a, c, st, bps);
-    case 32: return launch_planned_one<FT, VT, NM, 32, V>(a, c, st, bps);
+    case 2: return launch_planned_one<FT, VT, NM, 2, V, 1, PHI>(a, c, st, bps);
+    case 4: return launch_planned_one<FT, VT, NM, 4, V, 1, PHI>(a, c, st, bps);
+    case 8: return launch_planned_one<FT, VT, NM, 8, V, 1, PHI>(a, c, st, bps);
+    case 16: return launch_planned_one<FT, VT, NM, 16, V, 1, PHI>(a, c, st, bps);
+    case 32: return launch_planned_one<FT, VT, NM, 32, V, 1, PHI>(a, c, st, bps);
     }
     return fail(ALTOB_ERR_UNSUPPORTED, "lanes per nonzero");
 }
@@ -153,7 +163,7 @@ altob_status launch_planned_batch_one(const BatchTiles<FT>& bt, const TiledCfg& 
 {
     static std::atomic<size_t> configured{0};
     constexpr int V = 16 / sizeof(FT);
-    constexpr int mb = planned_min_blocks<FT, NM, LPN>();
+    constexpr int mb = planned_min_blocks<FT, NM, LPN, 1, false>();
     if constexpr (mb > 0)
         return launch_kernel(k_planned_batch_mb<FT, VT, NM, LPN, V, mb>, configured, &bt, c, st, bps);
     else
@@ -229,9 +239,12 @@ altob_status launch_batch_shape(const BatchTiles<FT>& bt, const TiledCfg& c, cud
                                         int* bps)                                                      \
     {                                                                                                  \
         switch (a.nmode) {                                                                             \
-        case 3: return launch_planned_shape<FT, VT, 3>(a, c, st, bps);                                 \
-        case 4: return launch_planned_shape<FT, VT, 4>(a, c, st, bps);                                 \
-        case 5: return launch_planned_shape<FT, VT, 5>(a, c, st, bps);                                 \
+        case 3: return c.phi ? launch_planned_shape<FT, VT, 3, true>(a, c, st, bps)                    \
+                             : launch_planned_shape<FT, VT, 3, false>(a, c, st, bps);                  \
+        case 4: return c.phi ? launch_planned_shape<FT, VT, 4, true>(a, c, st, bps)                    \
+                             : launch_planned_shape<FT, VT, 4, false>(a, c, st, bps);                  \
+        case 5: return c.phi ? launch_planned_shape<FT, VT, 5, true>(a, c, st, bps)                    \
+                             : launch_planned_shape<FT, VT, 5, false>(a, c, st, bps);                  \
         }                                                                                              \
         return fail(ALTOB_ERR_UNSUPPORTED, "planned kernel: order 3-5");                               \
     }                                                                                                  \
