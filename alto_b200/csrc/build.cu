@@ -2,11 +2,11 @@
 //
 // Replaces create_alto (IntelLabs/ALTO include/alto.hpp:108-294):
 //   setup_packed_alto  (alto.hpp:669-770)  -> host, make_masks()
-//   pdep linearization (alto.hpp:184-202)  -> k_linearize (expand network)
-//   sort_alto          (alto.hpp:772-803)  -> radix_sort_pairs (LSD, 8-bit digits)
+//   pdep linearization (alto.hpp:184-202)  -> k_linearize (field layout), digits gathered in the sort
+//   sort_alto          (alto.hpp:772-803)  -> alto_sort (radix.cu)
 //   oidx               (alto.hpp:246-285)  -> radix sort of mode indices
 //   prtn_alto          (alto.hpp:805-899)  -> k_intervals
-//   CR bits            (alto.hpp:930-1027) -> k_cr_owner + k_cr_set
+//   CR bits            (alto.hpp:930-1027) -> k_cr_shared + k_cr_set
 #include <algorithm>
 #include <cstdio>
 #include <cstring>
@@ -191,269 +191,49 @@ Decoder make_decoder(int nmode, const u128* masks, int alto_bits)
     return d;
 }
 
-// ----------------------------------------------------------- scans
-// Exclusive prefix sum of u32 values in place (sum < 2^32).
-
-static constexpr int SC_THREADS = 1024;
-static constexpr int SC_IPT = 4;
-static constexpr int SC_CHUNK = SC_THREADS * SC_IPT;
-
-__device__ __forceinline__ u32 block_excl_scan(u32 v, u32* total, u32* warp_sums)
-{
-    int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    u32 x = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        u32 y = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= o) x += y;
-    }
-    if (lane == 31) warp_sums[warp] = x;
-    __syncthreads();
-    if (warp == 0) {
-        u32 s = lane < nw ? warp_sums[lane] : 0;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            u32 y = __shfl_up_sync(0xffffffffu, s, o);
-            if (lane >= o) s += y;
-        }
-        if (lane < nw) warp_sums[lane] = s;
-    }
-    __syncthreads();
-    u32 base = warp ? warp_sums[warp - 1] : 0;
-    *total = warp_sums[nw - 1];
-    __syncthreads();
-    return base + x - v;
-}
-
-__global__ void k_scan_reduce(const u32* in, u64 n, u32* bsum)
-{
-    __shared__ u32 ws[32];
-    u64 base = (u64)blockIdx.x * SC_CHUNK + (u64)threadIdx.x * SC_IPT;
-    u32 s = 0;
-#pragma unroll
-    for (int k = 0; k < SC_IPT; ++k)
-        if (base + k < n) s += in[base + k];
-    u32 tot;
-    block_excl_scan(s, &tot, ws);
-    if (threadIdx.x == 0) bsum[blockIdx.x] = tot;
-}
-
-__global__ void k_scan_top(u32* bsum, u32 nb)
-{
-    __shared__ u32 ws[32];
-    u32 carry = 0;
-    for (u32 b0 = 0; b0 < nb; b0 += blockDim.x) {
-        u32 i = b0 + threadIdx.x;
-        u32 v = i < nb ? bsum[i] : 0;
-        u32 tot;
-        u32 ex = block_excl_scan(v, &tot, ws);
-        if (i < nb) bsum[i] = carry + ex;
-        carry += tot;
-    }
-}
-
-__global__ void k_scan_down(u32* data, u64 n, const u32* bsum)
-{
-    __shared__ u32 ws[32];
-    u64 base = (u64)blockIdx.x * SC_CHUNK + (u64)threadIdx.x * SC_IPT;
-    u32 v[SC_IPT];
-    u32 s = 0;
-#pragma unroll
-    for (int k = 0; k < SC_IPT; ++k) {
-        v[k] = base + k < n ? data[base + k] : 0;
-        s += v[k];
-    }
-    u32 tot;
-    u32 ex = block_excl_scan(s, &tot, ws) + bsum[blockIdx.x];
-#pragma unroll
-    for (int k = 0; k < SC_IPT; ++k) {
-        if (base + k < n) data[base + k] = ex;
-        ex += v[k];
-    }
-}
-
-static altob_status excl_scan_u32(u32* data, u64 n, u32* bsum, cudaStream_t st)
-{
-    u32 nb = (u32)((n + SC_CHUNK - 1) / SC_CHUNK);
-    if (nb == 0) return ALTOB_OK;
-    k_scan_reduce<<<nb, SC_THREADS, 0, st>>>(data, n, bsum);
-    ALTOB_LAUNCH_CHECK();
-    k_scan_top<<<1, SC_THREADS, 0, st>>>(bsum, nb);
-    ALTOB_LAUNCH_CHECK();
-    k_scan_down<<<nb, SC_THREADS, 0, st>>>(data, n, bsum);
-    ALTOB_LAUNCH_CHECK();
-    return ALTOB_OK;
-}
-
-// ------------------------------------------------------- radix sort
-// LSD radix sort, 8-bit digits.  Per pass: tile histograms (digit-major),
-// one exclusive scan, then a stable scatter in which every tile ranks its
-// keys with warp match + a per-round scan over the eight warps.
-
-static constexpr int RS_THREADS = 256;
-static constexpr int RS_IPT = 16;
-static constexpr int RS_TILE = RS_THREADS * RS_IPT;
-static constexpr int RS_WARPS = RS_THREADS / 32;
-
-template <int KW>
-__device__ __forceinline__ u32 rs_digit(u64 lo, u64 hi, int shift)
-{
-    u64 w = (KW == 2 && shift >= 64) ? hi : lo;
-    return (u32)(w >> (shift & 63)) & 0xffu;
-}
-
-template <int KW>
-__global__ void __launch_bounds__(RS_THREADS) k_rs_hist(const u64* __restrict__ klo, const u64* __restrict__ khi,
-                                                        u64 n, int shift, u32* __restrict__ hist, u32 ntiles)
-{
-    __shared__ u32 h[RS_WARPS][256];
-    for (int j = threadIdx.x; j < RS_WARPS * 256; j += RS_THREADS) (&h[0][0])[j] = 0;
-    __syncthreads();
-    int warp = threadIdx.x >> 5;
-    u64 base = (u64)blockIdx.x * RS_TILE;
-#pragma unroll 4
-    for (int k = 0; k < RS_IPT; ++k) {
-        u64 i = base + (u64)k * RS_THREADS + threadIdx.x;
-        if (i < n) {
-            u64 lo = (KW == 1 || shift < 64) ? klo[i] : 0;
-            u64 hi = (KW == 2 && shift >= 64) ? khi[i] : 0;
-            atomicAdd(&h[warp][rs_digit<KW>(lo, hi, shift)], 1u);
-        }
-    }
-    __syncthreads();
-    u32 d = threadIdx.x;
-    u32 s = 0;
-#pragma unroll
-    for (int w = 0; w < RS_WARPS; ++w) s += h[w][d];
-    hist[(u64)d * ntiles + blockIdx.x] = s;
-}
-
-template <int KW>
-__global__ void __launch_bounds__(RS_THREADS) k_rs_scatter(const u64* __restrict__ klo, const u64* __restrict__ khi,
-                                                           const u32* __restrict__ pay, u64* __restrict__ olo,
-                                                           u64* __restrict__ ohi, u32* __restrict__ opay, u64 n,
-                                                           int shift, const u32* __restrict__ offs, u32 ntiles)
-{
-    __shared__ u32 run[256];
-    __shared__ u32 wcnt[RS_WARPS][256];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    run[tid] = offs[(u64)tid * ntiles + blockIdx.x];
-    const u64 base = (u64)blockIdx.x * RS_TILE;
-    for (int k = 0; k < RS_IPT; ++k) {
-        const u64 i = base + (u64)k * RS_THREADS + tid;
-        const bool valid = i < n;
-        u64 lo = 0, hi = 0;
-        u32 p = 0, d = 256;
-        if (valid) {
-            lo = klo[i];
-            if (KW == 2) hi = khi[i];
-            p = pay[i];
-            d = rs_digit<KW>(lo, hi, shift);
-        }
-        for (int j = tid; j < RS_WARPS * 256; j += RS_THREADS) (&wcnt[0][0])[j] = 0;
-        __syncthreads();
-        const u32 peers = __match_any_sync(0xffffffffu, d);
-        const u32 rank = __popc(peers & ((1u << lane) - 1u));
-        if (valid && lane == __ffs(peers) - 1) wcnt[warp][d] = __popc(peers);
-        __syncthreads();
-        {
-            u32 r = run[tid];
-#pragma unroll
-            for (int w = 0; w < RS_WARPS; ++w) {
-                u32 c = wcnt[w][tid];
-                wcnt[w][tid] = r;
-                r += c;
-            }
-            run[tid] = r;
-        }
-        __syncthreads();
-        if (valid) {
-            u32 dst = wcnt[warp][d] + rank;
-            olo[dst] = lo;
-            if (KW == 2) ohi[dst] = hi;
-            opay[dst] = p;
-        }
-        __syncthreads();
-    }
-}
-
-altob_status radix_sort_pairs(u64* klo, u64* khi, u32* pay, u64* klo_alt, u64* khi_alt, u32* pay_alt, u64 n,
-                              int kw, int nbits, cudaStream_t st, bool* result_in_alt)
-{
-    *result_in_alt = false;
-    if (n <= 1 || nbits <= 0) return ALTOB_OK;
-    u32 ntiles = (u32)((n + RS_TILE - 1) / RS_TILE);
-    u64 hn = (u64)ntiles * 256;
-    u32* hist = nullptr;
-    u32* bsum = nullptr;
-    ALTOB_TRY(dmalloc_t(&hist, hn));
-    altob_status s = dmalloc_t(&bsum, hn / SC_CHUNK + 2);
-    if (s != ALTOB_OK) {
-        dfree(hist);
-        return s;
-    }
-    bool alt = false;
-    for (int shift = 0; shift < nbits; shift += 8) {
-        u64* slo = alt ? klo_alt : klo;
-        u64* shi = alt ? khi_alt : khi;
-        u32* sp = alt ? pay_alt : pay;
-        u64* dlo = alt ? klo : klo_alt;
-        u64* dhi = alt ? khi : khi_alt;
-        u32* dp = alt ? pay : pay_alt;
-        if (kw == 2) {
-            k_rs_hist<2><<<ntiles, RS_THREADS, 0, st>>>(slo, shi, n, shift, hist, ntiles);
-        } else {
-            k_rs_hist<1><<<ntiles, RS_THREADS, 0, st>>>(slo, shi, n, shift, hist, ntiles);
-        }
-        s = excl_scan_u32(hist, hn, bsum, st);
-        if (s != ALTOB_OK) break;
-        if (kw == 2) {
-            k_rs_scatter<2><<<ntiles, RS_THREADS, 0, st>>>(slo, shi, sp, dlo, dhi, dp, n, shift, hist, ntiles);
-        } else {
-            k_rs_scatter<1><<<ntiles, RS_THREADS, 0, st>>>(slo, shi, sp, dlo, dhi, dp, n, shift, hist, ntiles);
-        }
-        cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) {
-            s = fail(ALTOB_ERR_CUDA, std::string("radix scatter: ") + cudaGetErrorString(e));
-            break;
-        }
-        alt = !alt;
-    }
-    cudaStreamSynchronize(st);
-    dfree(hist);
-    dfree(bsum);
-    *result_in_alt = alt;
-    return s;
-}
-
 // ------------------------------------------------------ build kernels
 
-// pdep linearization: key = OR over modes of expand(coord, mask).  Also
-// validates every coordinate against its dimension.
-__global__ void k_linearize(const u64* __restrict__ cidx, u64 nnz, Decoder dec, u64 dmax0, u64 dmax1, u64 dmax2,
-                            u64 dmax3, u64 dmax4, int kw, u64* __restrict__ klo, u64* __restrict__ khi,
-                            u32* __restrict__ perm, int* __restrict__ bad)
+// Linearization (alto.hpp:184-202) straight into the device's field layout:
+// every mode index at its bit field, bits past 64 in `hi` (HI wide, or none).
+// The ALTO order of these keys is read off them digit by digit when they are
+// sorted.  Also validates every coordinate against its dimension.
+struct DimMax {
+    u64 d[ALTOB_MAX_MODES];
+};
+
+template <typename HI>
+__global__ void __launch_bounds__(256) k_linearize(const u64* __restrict__ cidx, u64 nnz, Fields f, DimMax dm,
+                                                   u64* __restrict__ klo, HI* __restrict__ khi, int* __restrict__ bad)
 {
-    const u64 dm[5] = {dmax0, dmax1, dmax2, dmax3, dmax4};
     for (u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x; i < nnz; i += (u64)gridDim.x * blockDim.x) {
-        u32 w[4] = {0, 0, 0, 0};
-        for (int m = 0; m < dec.nmode; ++m) {
-            u64 c64 = cidx[(u64)m * nnz + i];
-            if (c64 >= dm[m]) {
-                atomicExch(bad, 1);
-                c64 = 0;
-            }
-            u32 c = (u32)c64;
+        u64 lo = 0, hi = 0;
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const WordDec& wd = dec.md[m].w[q];
-                if (q < dec.nwords && wd.m) w[q] |= expand32(c >> wd.off, wd);
+        for (int m = 0; m < ALTOB_MAX_MODES; ++m) {
+            if (m >= f.nmode) break;
+            u64 c = cidx[(u64)m * nnz + i];
+            if (c >= dm.d[m]) {
+                atomicExch(bad, 1);
+                c = 0;
+            }
+            const u32 p = f.pos[m];
+            if (p < 64) {
+                lo |= c << p;
+                if (p > 32) hi |= c >> (64 - p);
+            } else {
+                hi |= c << (p - 64);
             }
         }
-        klo[i] = (u64)w[0] | ((u64)w[1] << 32);
-        if (kw == 2) khi[i] = (u64)w[2] | ((u64)w[3] << 32);
-        perm[i] = (u32)i;
+        klo[i] = lo;
+        if (khi) khi[i] = (HI)hi;
     }
+}
+
+// The high words of a sort as explicit 64-bit words.
+template <typename HI>
+__global__ void k_widen_hi(const HI* __restrict__ in, u64 n, u64* __restrict__ out)
+{
+    for (u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (u64)gridDim.x * blockDim.x)
+        out[i] = in ? (u64)in[i] : 0;
 }
 
 template <typename VI, typename VO>
@@ -461,29 +241,6 @@ __global__ void k_gather_vals(const VI* __restrict__ in, const u32* __restrict__
 {
     for (u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (u64)gridDim.x * blockDim.x)
         out[i] = (VO)in[perm[i]];
-}
-
-// Interleaved ALTO key -> field layout (same sort order).  CR bits are not
-// set yet at this point.
-__global__ void k_reencode(u64* __restrict__ klo, u64* __restrict__ khi, int kw, u64 n, Decoder dec, Fields f)
-{
-    for (u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (u64)gridDim.x * blockDim.x) {
-        u32 w[4];
-        split_key(klo[i], kw == 2 ? khi[i] : 0ull, w);
-        u64 lo = 0, hi = 0;
-        for (int m = 0; m < dec.nmode; ++m) {
-            const u64 c = decode_mode(w, dec.md[m], dec.nwords);
-            const u32 p = f.pos[m];
-            if (p < 64) {
-                lo |= c << p;
-                if (p > 0 && p + 32 > 64) hi |= c >> (64 - p);
-            } else {
-                hi |= c << (p - 64);
-            }
-        }
-        klo[i] = lo;
-        if (kw == 2) khi[i] = hi;
-    }
 }
 
 // Field layout -> interleaved ALTO key (for altob_dump); bits at and above
@@ -512,13 +269,12 @@ __global__ void k_interleave(const u64* __restrict__ klo, KeySrc ks, int alto_bi
 }
 
 // Mode indices of the sorted keys (for the oidx sort).
-__global__ void k_mode_keys(const u64* __restrict__ klo, const u64* __restrict__ khi, u64 n, Fields f, int mode,
-                            u64* __restrict__ out, u32* __restrict__ iota)
+template <typename HI>
+__global__ void k_mode_keys(const u64* __restrict__ klo, const HI* __restrict__ khi, u64 n, Fields f, int mode,
+                            u32* __restrict__ out)
 {
-    for (u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (u64)gridDim.x * blockDim.x) {
-        out[i] = field(klo[i], khi ? khi[i] : 0ull, f.pos[mode], f.mask[mode]);
-        iota[i] = (u32)i;
-    }
+    for (u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (u64)gridDim.x * blockDim.x)
+        out[i] = field(klo[i], khi ? (u64)khi[i] : 0ull, f.pos[mode], f.mask[mode]);
 }
 
 __global__ void k_init_intervals(u64* iv, int nprtn, int nmode, u64 d0, u64 d1, u64 d2, u64 d3, u64 d4)
@@ -532,39 +288,52 @@ __global__ void k_init_intervals(u64* iv, int nprtn, int nmode, u64 d0, u64 d1, 
 }
 
 // Per-partition min / max of every mode index (prtn_alto, alto.hpp:874-899).
-// A warp whose 32 keys lie in one partition reduces in registers first.
-__global__ void k_intervals(const u64* __restrict__ klo, const u64* __restrict__ khi, u64 n, Fields f, u64 per,
-                            u64* __restrict__ iv)
+// A warp walks IV_CHUNK consecutive keys, keeps the extremes of the current
+// partition in registers and adds them to the table once per partition it
+// meets (one atomic pair per 32 keys took 452 us on 20.2M keys).
+constexpr u64 IV_CHUNK = 1024;
+
+template <typename HI>
+__global__ void __launch_bounds__(256) k_intervals(const u64* __restrict__ klo, const HI* __restrict__ khi, u64 n,
+                                                   Fields f, u64 per, u64* __restrict__ iv)
 {
     const int lane = threadIdx.x & 31;
-    const u64 stride = (u64)gridDim.x * blockDim.x;
-    for (u64 base = (u64)blockIdx.x * blockDim.x + (threadIdx.x & ~31u); base < n; base += stride) {
-        u64 i = base + lane;
-        bool valid = i < n;
-        u64 p = valid ? i / per : ~0ull;
-        u64 p0 = __shfl_sync(0xffffffffu, p, 0);
-        u64 pl = __shfl_sync(0xffffffffu, p, 31);
-        bool uniform = (p0 == pl) || (base + 31 >= n && __all_sync(0xffffffffu, !valid || p == p0));
-        u64 lo = valid ? klo[i] : 0, hi = (valid && khi) ? khi[i] : 0;
-        for (int m = 0; m < f.nmode; ++m) {
-            u32 c = valid ? field(lo, hi, f.pos[m], f.mask[m]) : 0;
-            if (uniform) {
-                u32 mn = valid ? c : 0xffffffffu, mx = valid ? c : 0;
+    const u64 nw = ((u64)gridDim.x * blockDim.x) >> 5;
+    for (u64 c = ((u64)blockIdx.x * blockDim.x + threadIdx.x) >> 5; c * IV_CHUNK < n; c += nw) {
+        u64 i0 = c * IV_CHUNK;
+        const u64 stop = min(n, i0 + IV_CHUNK);
+        u64 p = i0 / per;
+        while (i0 < stop) {
+            const u64 seg = min(stop, (p + 1) * per);
+            u32 mn[ALTOB_MAX_MODES], mx[ALTOB_MAX_MODES];
 #pragma unroll
-                for (int o = 16; o; o >>= 1) {
-                    mn = min(mn, __shfl_xor_sync(0xffffffffu, mn, o));
-                    mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-                }
-                if (lane == 0) {
-                    u64* e = iv + (p0 * f.nmode + m) * 2;
-                    atomicMin((unsigned long long*)e, (unsigned long long)mn);
-                    atomicMax((unsigned long long*)(e + 1), (unsigned long long)mx);
-                }
-            } else if (valid) {
-                u64* e = iv + (p * f.nmode + m) * 2;
-                atomicMin((unsigned long long*)e, (unsigned long long)c);
-                atomicMax((unsigned long long*)(e + 1), (unsigned long long)c);
+            for (int m = 0; m < ALTOB_MAX_MODES; ++m) {
+                mn[m] = 0xffffffffu;
+                mx[m] = 0;
             }
+#pragma unroll 4
+            for (u64 i = i0 + lane; i < seg; i += 32) {
+                const u64 lo = klo[i], hi = khi ? (u64)khi[i] : 0;
+#pragma unroll
+                for (int m = 0; m < ALTOB_MAX_MODES; ++m) {
+                    if (m >= f.nmode) break;
+                    const u32 x = field(lo, hi, f.pos[m], f.mask[m]);
+                    mn[m] = min(mn[m], x);
+                    mx[m] = max(mx[m], x);
+                }
+            }
+#pragma unroll
+            for (int m = 0; m < ALTOB_MAX_MODES; ++m) {
+                if (m >= f.nmode) break;
+                const u32 a = __reduce_min_sync(0xffffffffu, mn[m]), b = __reduce_max_sync(0xffffffffu, mx[m]);
+                if (lane == 0) {
+                    u64* e = iv + (p * f.nmode + m) * 2;
+                    atomicMin((unsigned long long*)e, (unsigned long long)a);
+                    atomicMax((unsigned long long*)(e + 1), (unsigned long long)b);
+                }
+            }
+            i0 = seg;
+            ++p;
         }
     }
 }
@@ -574,27 +343,29 @@ struct CrArgs {
     int bitpos[ALTOB_MAX_MODES];  // -1 = no CR bit for this mode
 };
 
-// Fiber ownership (alto.hpp:970-996): 0 untouched, p+1 one partition, -1 shared.
-__global__ void k_cr_owner(const u64* __restrict__ klo, const u64* __restrict__ khi, u64 n, Fields f, u64 per,
-                           CrArgs a)
+// Fibers that several partitions share (alto.hpp:970-996), from the mode's
+// sorted order: a fiber's nonzeros stand together with ascending positions,
+// so it is shared iff two neighbours lie in different partitions.  (Claiming
+// owners with one compare-and-swap per nonzero took 3558 us on 20.2M
+// nonzeros, serialised on the head rows.)
+__global__ void k_cr_shared(const u32* __restrict__ key, const u32* __restrict__ pos, u64 n, u32 per,
+                            int* __restrict__ owner)
 {
-    for (u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (u64)gridDim.x * blockDim.x) {
-        const u64 lo = klo[i], hi = khi ? khi[i] : 0;
-        int p1 = (int)(i / per) + 1;
-        for (int m = 0; m < f.nmode; ++m) {
-            if (a.bitpos[m] < 0) continue;
-            u32 c = field(lo, hi, f.pos[m], f.mask[m]);
-            int old = atomicCAS(&a.owner[m][c], 0, p1);
-            if (old != 0 && old != p1 && old != -1) atomicExch(&a.owner[m][c], -1);
-        }
+    for (u64 k = (u64)blockIdx.x * blockDim.x + threadIdx.x; k + 1 < n; k += (u64)gridDim.x * blockDim.x) {
+        const u32 c = key[k];
+        if (c == key[k + 1] && pos[k] / per != pos[k + 1] / per) owner[c] = -1;
     }
 }
 
-// Sets the CR bits of nonzeros whose fiber is shared (alto.hpp:998-1019).
-__global__ void k_cr_set(u64* __restrict__ klo, u64* __restrict__ khi, u64 n, Fields f, CrArgs a)
+// Sets the CR bits of nonzeros whose fiber is shared (alto.hpp:998-1019) in
+// klo and the explicit high words khi (if any); src holds the high words the
+// mode indices are read from.
+template <typename HI>
+__global__ void k_cr_set(u64* __restrict__ klo, u64* __restrict__ khi, u64 n, Fields f, CrArgs a,
+                         const HI* __restrict__ src)
 {
     for (u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (u64)gridDim.x * blockDim.x) {
-        const u64 lo = klo[i], hi = khi ? khi[i] : 0;
+        const u64 lo = klo[i], hi = src ? (u64)src[i] : 0;
         u64 add_lo = 0, add_hi = 0;
         for (int m = 0; m < f.nmode; ++m) {
             int b = a.bitpos[m];
@@ -611,12 +382,15 @@ __global__ void k_cr_set(u64* __restrict__ klo, u64* __restrict__ khi, u64 n, Fi
 }
 
 // Positions where the high key word changes (for the run table) and a
-// check that it never decreases.
-__global__ void k_hi_runs(const u64* __restrict__ khi, u64 n, u64* __restrict__ starts, u32 cap,
+// check that it never decreases; either outcome that rules the table out ends
+// the search.
+template <typename HI>
+__global__ void k_hi_runs(const HI* __restrict__ khi, u64 n, u64* __restrict__ starts, u32 cap,
                           u32* __restrict__ count, u32* __restrict__ decreasing)
 {
     for (u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (u64)gridDim.x * blockDim.x) {
         if (i == 0 || khi[i] != khi[i - 1]) {
+            if (*(volatile u32*)decreasing || *(volatile u32*)count > cap) return;
             if (i > 0 && khi[i] < khi[i - 1]) atomicExch(decreasing, 1u);
             u32 k = atomicAdd(count, 1u);
             if (k < cap) starts[k] = i;
@@ -624,9 +398,10 @@ __global__ void k_hi_runs(const u64* __restrict__ khi, u64 n, u64* __restrict__ 
     }
 }
 
-__global__ void k_gather_u64(const u64* __restrict__ src, const u64* __restrict__ idx, u32 n, u64* __restrict__ out)
+template <typename HI>
+__global__ void k_gather_hi(const HI* __restrict__ src, const u64* __restrict__ idx, u32 n, u64* __restrict__ out)
 {
-    for (u32 i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) out[i] = src[idx[i]];
+    for (u32 i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) out[i] = (u64)src[idx[i]];
 }
 
 // Explicit high key word of every nonzero of a tensor that keeps them as a
@@ -635,6 +410,12 @@ __global__ void k_expand_hi(KeySrc key, u64 n, u64* __restrict__ hi)
 {
     for (u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (u64)gridDim.x * blockDim.x)
         hi[i] = key_hi(key, i);
+}
+
+static int intervals_grid(u64 n)
+{
+    const u64 warps = (n + IV_CHUNK - 1) / IV_CHUNK;
+    return (int)std::max<u64>(1, std::min<u64>((warps + 7) / 8, (u64)num_sms() * 8));
 }
 
 static int grid_for(u64 n, int threads)
@@ -646,25 +427,34 @@ static int grid_for(u64 n, int threads)
 
 // ------------------------------------------------------------ create
 
-static altob_status build(altob_tensor* t, const u64* d_cidx, const void* d_vals_in, altob_dtype vin,
+// HI: the type the key bits past 64 have while they are sorted (hi_bytes
+// wide; 0: the keys fit 64 bits).
+template <typename HI>
+static altob_status build(altob_tensor* t, const u64* d_cidx, const void* d_vals_in, altob_dtype vin, int hi_bytes,
                           cudaStream_t st)
 {
     const u64 nnz = t->nnz;
-    const int kw = t->kw;
-    u64 *klo = nullptr, *khi = nullptr, *klo2 = nullptr, *khi2 = nullptr;
+    u64 *klo = nullptr, *klo2 = nullptr, *khi64 = nullptr, *starts = nullptr, *d_iv = nullptr;
+    HI *khi = nullptr, *khi2 = nullptr;
     u32 *perm = nullptr, *perm2 = nullptr;
-    int* bad = nullptr;
+    u32* flags = nullptr;  // a coordinate out of range | high-word runs | a high word decreases
+    CrArgs ca;
+    memset(&ca, 0, sizeof(ca));
     altob_status s = ALTOB_OK;
     auto cleanup = [&] {
-        cudaStreamSynchronize(st);
         dfree(klo2);
+        dfree(khi);
         dfree(khi2);
         dfree(perm);
         dfree(perm2);
-        dfree(bad);
+        dfree(flags);
+        dfree(starts);
+        dfree(d_iv);
+        for (int n = 0; n < ALTOB_MAX_MODES; ++n) dfree(ca.owner[n]);
         if (s != ALTOB_OK) {
             dfree(klo);
-            dfree(khi);
+            dfree(khi64);
+            cudaStreamSynchronize(st);  // the caller's arrays are not read after the return
         }
     };
 #define BTRY(x)             \
@@ -675,46 +465,42 @@ static altob_status build(altob_tensor* t, const u64* d_cidx, const void* d_vals
             return s;       \
         }                   \
     } while (0)
+#define BLAUNCH(what)                                                                             \
+    do {                                                                                          \
+        const cudaError_t e_ = cudaGetLastError();                                                \
+        if (e_ != cudaSuccess)                                                                    \
+            BTRY(fail(ALTOB_ERR_CUDA, std::string(what " launch: ") + cudaGetErrorString(e_)));   \
+    } while (0)
+    const int grid = grid_for(nnz, 256);
     BTRY(dmalloc_t(&klo, nnz));
     BTRY(dmalloc_t(&klo2, nnz));
-    if (kw == 2) {
+    if (hi_bytes) {
         BTRY(dmalloc_t(&khi, nnz));
         BTRY(dmalloc_t(&khi2, nnz));
     }
     BTRY(dmalloc_t(&perm, nnz));
     BTRY(dmalloc_t(&perm2, nnz));
-    BTRY(dmalloc_t(&bad, 1));
-    cudaMemsetAsync(bad, 0, sizeof(int), st);
-    u64 dm[5] = {1, 1, 1, 1, 1};
-    for (int n = 0; n < t->nmode; ++n) dm[n] = t->dims[n];
+    BTRY(dmalloc_t(&flags, 3));
+    cudaMemsetAsync(flags, 0, 3 * sizeof(u32), st);
+    DimMax dm;
+    for (int n = 0; n < ALTOB_MAX_MODES; ++n) dm.d[n] = n < t->nmode ? t->dims[n] : 1;
     if (nnz) {
-        k_linearize<<<grid_for(nnz, 256), 256, 0, st>>>(d_cidx, nnz, t->dec, dm[0], dm[1], dm[2], dm[3], dm[4], kw,
-                                                        klo, khi, perm, bad);
-        if (cudaGetLastError() != cudaSuccess) BTRY(fail(ALTOB_ERR_CUDA, "k_linearize launch failed"));
-        int hbad = 0;
-        cudaMemcpyAsync(&hbad, bad, sizeof(int), cudaMemcpyDeviceToHost, st);
-        if (cudaStreamSynchronize(st) != cudaSuccess) BTRY(fail(ALTOB_ERR_CUDA, "linearize failed"));
-        if (hbad) BTRY(fail(ALTOB_ERR_ARG, "a coordinate is not below its dimension"));
+        k_linearize<HI><<<grid, 256, 0, st>>>(d_cidx, nnz, t->fld, dm, klo, khi, (int*)flags);
+        BLAUNCH("k_linearize");
     }
     bool in_alt = false;
-    BTRY(radix_sort_pairs(klo, khi, perm, klo2, khi2, perm2, nnz, kw, t->alto_bits, st, &in_alt));
+    BTRY(alto_sort(klo, khi, perm, klo2, khi2, perm2, nnz, hi_bytes, t->masks, t->fld, t->alto_bits, st, &in_alt));
     if (in_alt) {
         std::swap(klo, klo2);
         std::swap(khi, khi2);
         std::swap(perm, perm2);
     }
-    // interleaved -> field layout (same order)
-    if (nnz) {
-        k_reencode<<<grid_for(nnz, 256), 256, 0, st>>>(klo, khi, kw, nnz, t->dec, t->fld);
-        if (cudaGetLastError() != cudaSuccess) BTRY(fail(ALTOB_ERR_CUDA, "k_reencode launch failed"));
-    }
     // values in sorted order, converted to the stored dtype
     size_t vsz = val_size(t->vdt);
     BTRY(dmalloc(&t->d_vals, nnz * vsz + 16));
     if (nnz) {
-        int g = grid_for(nnz, 256);
 #define GATHER(VI, VO) \
-    k_gather_vals<VI, VO><<<g, 256, 0, st>>>((const VI*)d_vals_in, perm, nnz, (VO*)t->d_vals)
+    k_gather_vals<VI, VO><<<grid, 256, 0, st>>>((const VI*)d_vals_in, perm, nnz, (VO*)t->d_vals)
         if (vin == ALTOB_F64 && t->vdt == ALTOB_F64) GATHER(double, double);
         else if (vin == ALTOB_F64 && t->vdt == ALTOB_F32) GATHER(double, float);
         else if (vin == ALTOB_F32 && t->vdt == ALTOB_F32) GATHER(float, float);
@@ -723,65 +509,14 @@ static altob_status build(altob_tensor* t, const u64* d_cidx, const void* d_vals
         else if (vin == ALTOB_F64 && t->vdt == ALTOB_U32) GATHER(double, u32);
         else BTRY(fail(ALTOB_ERR_UNSUPPORTED, "value dtype conversion not supported"));
 #undef GATHER
-        if (cudaGetLastError() != cudaSuccess) BTRY(fail(ALTOB_ERR_CUDA, "gather launch failed"));
+        BLAUNCH("k_gather_vals");
     }
 
-    // oidx for low-reuse modes (alto.hpp:246-285)
-    t->is_oidx = 0;
-    for (int n = 0; n < t->nmode; ++n)
-        if (fib_reuse(t, n) <= 4) t->is_oidx = 1;
-    if (t->is_oidx && nnz) {
-        for (int n = 0; n < t->nmode; ++n) {
-            if (fib_reuse(t, n) > 4) continue;
-            // klo2 / perm2 are free at this point: mode keys + iota
-            u64* mk = klo2;
-            u64* mk2 = nullptr;
-            u32* ox2 = nullptr;
-            BTRY(dmalloc_t(&mk2, nnz));
-            s = dmalloc_t(&ox2, nnz);
-            if (s != ALTOB_OK) {
-                dfree(mk2);
-                cleanup();
-                return s;
-            }
-            k_mode_keys<<<grid_for(nnz, 256), 256, 0, st>>>(klo, khi, nnz, t->fld, n, mk, perm2);
-            bool alt2 = false;
-            s = radix_sort_pairs(mk, nullptr, perm2, mk2, nullptr, ox2, nnz, 1, mode_bits(t->dims[n]), st, &alt2);
-            dfree(mk2);
-            if (s != ALTOB_OK) {
-                dfree(ox2);
-                cleanup();
-                return s;
-            }
-            if (alt2) {
-                t->d_oidx[n] = ox2;
-            } else {
-                t->d_oidx[n] = perm2;
-                perm2 = ox2;
-            }
-        }
-    }
-
-    // partitions (alto.hpp:822-836) and intervals (:874-899)
     const int np = t->nprtn, nm = t->nmode;
     const u64 per = (nnz + (u64)np - 1) / (u64)np;
-    t->prtn_ptr.assign(np + 1, 0);
-    for (int p = 0; p < np; ++p) t->prtn_ptr[p + 1] = std::min<u64>((u64)(p + 1) * per, nnz);
-    u64* d_iv = nullptr;
-    BTRY(dmalloc_t(&d_iv, (u64)np * nm * 2));
-    k_init_intervals<<<(np * nm + 255) / 256, 256, 0, st>>>(d_iv, np, nm, dm[0], dm[1], dm[2], dm[3], dm[4]);
-    if (nnz) k_intervals<<<grid_for(nnz, 256), 256, 0, st>>>(klo, khi, nnz, t->fld, per, d_iv);
-    t->intervals.assign((size_t)np * nm * 2, 0);
-    cudaMemcpyAsync(t->intervals.data(), d_iv, t->intervals.size() * sizeof(u64), cudaMemcpyDeviceToHost, st);
-    cudaError_t e = cudaStreamSynchronize(st);
-    dfree(d_iv);
-    if (e != cudaSuccess) BTRY(fail(ALTOB_ERR_CUDA, std::string("intervals: ") + cudaGetErrorString(e)));
-
-    // CR bits (alto.hpp:932-1027)
-    CrArgs ca;
-    memset(&ca, 0, sizeof(ca));
+    // which modes get CR bits (alto.hpp:932-968): all of them have an oidx
     int free_bits = t->lit_bits - t->alto_bits;
-    bool any_cr = false;
+    bool any_cr = false, cr_hi = false;
     t->alto_cr_mask = 0;
     for (int n = 0; n < nm; ++n) {
         ca.bitpos[n] = -1;
@@ -793,81 +528,115 @@ static altob_status build(altob_tensor* t, const u64* d_cidx, const void* d_vals
             t->alto_cr_mask |= t->cr_masks[n];
             --free_bits;
             any_cr = true;
+            cr_hi = cr_hi || b >= 64;
         }
     }
+    // oidx for low-reuse modes (alto.hpp:246-285)
+    t->is_oidx = 0;
+    for (int n = 0; n < t->nmode; ++n)
+        if (fib_reuse(t, n) <= 4) t->is_oidx = 1;
+    if (t->is_oidx && nnz) {
+        for (int n = 0; n < t->nmode; ++n) {
+            if (fib_reuse(t, n) > 4) continue;
+            // klo2 / perm2 are free at this point: two 32-bit key arrays, one payload
+            u32 *mk = (u32*)klo2, *ox2 = nullptr;
+            BTRY(dmalloc_t(&ox2, nnz));
+            k_mode_keys<HI><<<grid, 256, 0, st>>>(klo, khi, nnz, t->fld, n, mk);
+            bool alt2 = false;
+            s = radix_argsort_u32(mk, perm2, mk + nnz, ox2, nnz, mode_bits(t->dims[n]), st, &alt2);
+            if (s == ALTOB_OK && ca.bitpos[n] >= 0) s = dmalloc_t(&ca.owner[n], t->dims[n]);
+            if (s != ALTOB_OK) {
+                dfree(ox2);
+                cleanup();
+                return s;
+            }
+            if (ca.bitpos[n] >= 0) {
+                cudaMemsetAsync(ca.owner[n], 0, t->dims[n] * sizeof(int), st);
+                k_cr_shared<<<grid, 256, 0, st>>>(alt2 ? mk + nnz : mk, alt2 ? ox2 : perm2, nnz, (u32)per, ca.owner[n]);
+                BLAUNCH("k_cr_shared");
+            }
+            if (alt2) {
+                t->d_oidx[n] = ox2;
+            } else {
+                t->d_oidx[n] = perm2;
+                perm2 = ox2;
+            }
+        }
+    }
+
+    // partitions (alto.hpp:822-836) and intervals (:874-899)
+    t->prtn_ptr.assign(np + 1, 0);
+    for (int p = 0; p < np; ++p) t->prtn_ptr[p + 1] = std::min<u64>((u64)(p + 1) * per, nnz);
+    BTRY(dmalloc_t(&d_iv, (u64)np * nm * 2));
+    k_init_intervals<<<(np * nm + 255) / 256, 256, 0, st>>>(d_iv, np, nm, dm.d[0], dm.d[1], dm.d[2], dm.d[3], dm.d[4]);
+    if (nnz) k_intervals<HI><<<intervals_grid(nnz), 256, 0, st>>>(klo, khi, nnz, t->fld, per, d_iv);
+    BLAUNCH("k_intervals");
+    t->intervals.assign((size_t)np * nm * 2, 0);
+
     if (any_cr && nnz) {
-        for (int n = 0; n < nm; ++n) {
-            if (ca.bitpos[n] < 0) continue;
-            s = dmalloc_t(&ca.owner[n], t->dims[n]);
-            if (s == ALTOB_OK) cudaMemsetAsync(ca.owner[n], 0, t->dims[n] * sizeof(int), st);
-            if (s != ALTOB_OK) break;
+        if (cr_hi) {  // CR bits past 64: explicit high words
+            BTRY(dmalloc_t(&khi64, nnz));
+            k_widen_hi<HI><<<grid, 256, 0, st>>>(khi, nnz, khi64);
         }
-        if (s == ALTOB_OK) {
-            k_cr_owner<<<grid_for(nnz, 256), 256, 0, st>>>(klo, khi, nnz, t->fld, per, ca);
-            k_cr_set<<<grid_for(nnz, 256), 256, 0, st>>>(klo, khi, nnz, t->fld, ca);
-            e = cudaStreamSynchronize(st);
-            if (e != cudaSuccess) s = fail(ALTOB_ERR_CUDA, std::string("CR bits: ") + cudaGetErrorString(e));
-        }
-        for (int n = 0; n < nm; ++n) dfree(ca.owner[n]);
-        if (s != ALTOB_OK) {
-            cleanup();
-            return s;
-        }
+        k_cr_set<<<grid, 256, 0, st>>>(klo, khi64, nnz, t->fld, ca, khi);
+        BLAUNCH("CR bits");
     }
     // high key words: a run table when they never decrease along the stream
     // (the usual case: they are the top ALTO bits), else one word per nonzero
-    if (kw == 2 && nnz) {
-        const u32 cap = 1u << 16;
-        u64* starts = nullptr;
-        u32* cnt = nullptr;
+    const u32 cap = 1u << 16;
+    const bool has_hi = t->kw == 2 && nnz;
+    if (has_hi) {
         BTRY(dmalloc_t(&starts, cap));
-        s = dmalloc_t(&cnt, 2);
+        if (khi64) k_hi_runs<u64><<<grid, 256, 0, st>>>(khi64, nnz, starts, cap, flags + 1, flags + 2);
+        else k_hi_runs<HI><<<grid, 256, 0, st>>>(khi, nnz, starts, cap, flags + 1, flags + 2);
+        BLAUNCH("k_hi_runs");
+    }
+    // one wait for the whole build
+    u32 hf[3] = {0, 0, 0};
+    cudaMemcpyAsync(hf, flags, sizeof(hf), cudaMemcpyDeviceToHost, st);
+    cudaMemcpyAsync(t->intervals.data(), d_iv, t->intervals.size() * sizeof(u64), cudaMemcpyDeviceToHost, st);
+    cudaError_t e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess) BTRY(fail(ALTOB_ERR_CUDA, std::string("tensor build: ") + cudaGetErrorString(e)));
+    if (hf[0]) BTRY(fail(ALTOB_ERR_ARG, "a coordinate is not below its dimension"));
+    if (has_hi && hf[2] == 0 && hf[1] <= cap) {
+        std::vector<u64> hs(hf[1]);
+        cudaMemcpyAsync(hs.data(), starts, hf[1] * sizeof(u64), cudaMemcpyDeviceToHost, st);
+        cudaStreamSynchronize(st);
+        std::sort(hs.begin(), hs.end());
+        u64 *rs = nullptr, *rv = nullptr;
+        s = dmalloc_t(&rs, hf[1]);
+        if (s == ALTOB_OK) s = dmalloc_t(&rv, hf[1]);
+        if (s == ALTOB_OK) {
+            cudaMemcpyAsync(rs, hs.data(), hf[1] * sizeof(u64), cudaMemcpyHostToDevice, st);
+            const unsigned g = std::max(1u, (hf[1] + 255) / 256);
+            if (khi64) k_gather_hi<u64><<<g, 256, 0, st>>>(khi64, rs, hf[1], rv);
+            else k_gather_hi<HI><<<g, 256, 0, st>>>(khi, rs, hf[1], rv);
+            e = cudaStreamSynchronize(st);
+            if (e != cudaSuccess) s = fail(ALTOB_ERR_CUDA, std::string("high-word runs: ") + cudaGetErrorString(e));
+        }
         if (s != ALTOB_OK) {
-            dfree(starts);
+            dfree(rs);
+            dfree(rv);
             cleanup();
             return s;
         }
-        cudaMemsetAsync(cnt, 0, 2 * sizeof(u32), st);
-        k_hi_runs<<<grid_for(nnz, 256), 256, 0, st>>>(khi, nnz, starts, cap, cnt, cnt + 1);
-        u32 hc[2] = {0, 0};
-        cudaMemcpyAsync(hc, cnt, sizeof(hc), cudaMemcpyDeviceToHost, st);
+        t->d_run_start = rs;
+        t->d_run_val = rv;
+        t->nrun = (int)hf[1];
+        dfree(khi64);
+        khi64 = nullptr;
+    } else if (has_hi && !khi64) {
+        BTRY(dmalloc_t(&khi64, nnz));
+        k_widen_hi<HI><<<grid, 256, 0, st>>>(khi, nnz, khi64);
         e = cudaStreamSynchronize(st);
-        if (e == cudaSuccess && hc[1] == 0 && hc[0] <= cap) {
-            std::vector<u64> hs(hc[0]);
-            cudaMemcpyAsync(hs.data(), starts, hc[0] * sizeof(u64), cudaMemcpyDeviceToHost, st);
-            cudaStreamSynchronize(st);
-            std::sort(hs.begin(), hs.end());
-            u64 *rs = nullptr, *rv = nullptr;
-            s = dmalloc_t(&rs, hc[0]);
-            if (s == ALTOB_OK) s = dmalloc_t(&rv, hc[0]);
-            if (s == ALTOB_OK) {
-                cudaMemcpyAsync(rs, hs.data(), hc[0] * sizeof(u64), cudaMemcpyHostToDevice, st);
-                k_gather_u64<<<std::max(1u, (hc[0] + 255) / 256), 256, 0, st>>>(khi, rs, hc[0], rv);
-                e = cudaStreamSynchronize(st);
-                if (e == cudaSuccess) {
-                    t->d_run_start = rs;
-                    t->d_run_val = rv;
-                    t->nrun = (int)hc[0];
-                    dfree(khi);
-                    khi = nullptr;
-                } else {
-                    dfree(rs);
-                    dfree(rv);
-                }
-            } else {
-                dfree(rs);
-            }
-        }
-        dfree(starts);
-        dfree(cnt);
-        if (e != cudaSuccess) BTRY(fail(ALTOB_ERR_CUDA, std::string("high-word runs: ") + cudaGetErrorString(e)));
-        if (s != ALTOB_OK) BTRY(s);
+        if (e != cudaSuccess) BTRY(fail(ALTOB_ERR_CUDA, std::string("high words: ") + cudaGetErrorString(e)));
     }
     t->d_klo = klo;
-    t->d_khi = khi;
+    t->d_khi = khi64;
     cleanup();
 #undef BTRY
-    t->device_bytes = nnz * (8 * (khi ? 2 : 1) + vsz) + (u64)t->nrun * 16;
+#undef BLAUNCH
+    t->device_bytes = nnz * (8 * (t->d_khi ? 2 : 1) + vsz) + (u64)t->nrun * 16;
     for (int n = 0; n < nm; ++n)
         if (t->d_oidx[n]) t->device_bytes += nnz * 4;
     return ALTOB_OK;
@@ -925,7 +694,11 @@ static altob_status create_common(int nmode, const u64* dims, u64 nnz, const u64
             p += b;
         }
     }
-    altob_status s = build(t, d_cidx, d_vals, vdt, st);
+    const int hi_bits = total - 64;
+    altob_status s = hi_bits <= 0    ? build<unsigned char>(t, d_cidx, d_vals, vdt, 0, st)
+                     : hi_bits <= 8  ? build<unsigned char>(t, d_cidx, d_vals, vdt, 1, st)
+                     : hi_bits <= 32 ? build<u32>(t, d_cidx, d_vals, vdt, 4, st)
+                                     : build<u64>(t, d_cidx, d_vals, vdt, 8, st);
     if (s != ALTOB_OK) {
         altob_destroy(t);
         return s;
@@ -1025,7 +798,7 @@ static altob_status slice_impl(const altob_tensor* t, u64 begin, u64 end, int np
     if (s->is_oidx && n) {
         for (int m = 0; m < s->nmode; ++m) {
             if (fib_reuse(s, m) > 4) continue;
-            u64 *mk = nullptr, *mk2 = nullptr;
+            u32 *mk = nullptr, *mk2 = nullptr;
             u32 *io = nullptr, *io2 = nullptr;
             altob_status a = dmalloc_t(&mk, n);
             if (a == ALTOB_OK) a = dmalloc_t(&mk2, n);
@@ -1033,10 +806,10 @@ static altob_status slice_impl(const altob_tensor* t, u64 begin, u64 end, int np
             if (a == ALTOB_OK) a = dmalloc_t(&io2, n);
             bool alt = false;
             if (a == ALTOB_OK) {
-                k_mode_keys<<<grid_for(n, 256), 256, 0, st>>>(s->d_klo, hi, n, s->fld, m, mk, io);
+                k_mode_keys<u64><<<grid_for(n, 256), 256, 0, st>>>(s->d_klo, hi, n, s->fld, m, mk);
                 if (cudaGetLastError() != cudaSuccess) a = fail(ALTOB_ERR_CUDA, "k_mode_keys launch failed");
             }
-            if (a == ALTOB_OK) a = radix_sort_pairs(mk, nullptr, io, mk2, nullptr, io2, n, 1, mode_bits(s->dims[m]), st, &alt);
+            if (a == ALTOB_OK) a = radix_argsort_u32(mk, io, mk2, io2, n, mode_bits(s->dims[m]), st, &alt);
             dfree(mk);
             dfree(mk2);
             if (a == ALTOB_OK) {
@@ -1059,7 +832,7 @@ static altob_status slice_impl(const altob_tensor* t, u64 begin, u64 end, int np
     u64* d_iv = nullptr;
     ALTOB_TRY(dmalloc_t(&d_iv, (u64)np * nm * 2));
     k_init_intervals<<<(np * nm + 255) / 256, 256, 0, st>>>(d_iv, np, nm, dm[0], dm[1], dm[2], dm[3], dm[4]);
-    if (n) k_intervals<<<grid_for(n, 256), 256, 0, st>>>(s->d_klo, hi, n, s->fld, per, d_iv);
+    if (n) k_intervals<u64><<<intervals_grid(n), 256, 0, st>>>(s->d_klo, hi, n, s->fld, per, d_iv);
     s->intervals.assign((size_t)np * nm * 2, 0);
     cudaMemcpyAsync(s->intervals.data(), d_iv, s->intervals.size() * sizeof(u64), cudaMemcpyDeviceToHost, st);
     const cudaError_t e = cudaStreamSynchronize(st);

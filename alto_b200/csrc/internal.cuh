@@ -289,11 +289,32 @@ inline int env_int(const char* name, int dflt)
     return v && *v ? atoi(v) : dflt;
 }
 
-// Stable LSD radix sort of (key, payload) pairs on key bits [0, nbits).
-// Keys are kw u64 words (lo[], hi[]); payload is u32.  Ping-pong buffers
-// are provided by the caller; the result ends in the *_out arrays.
+// ---------------------------------------------------------- radix sorts
+// (radix.cu; stable, ping-pong buffers from the caller, the result is in the
+// *_alt arrays when *result_in_alt)
+
+// One 8-bit digit of a key: key bits [pos[0], pos[0] + 8) when pieces is 0,
+// else up to five bit fields (pos, mask); entry off[k] + v of the byte table
+// is the value v of piece k with its bits where the digit has them.  Pieces
+// of 8 bits in all take at most 256 entries.
+constexpr int KEY_DIGIT_LUT = 256;
+struct KeyDigit {
+    int pieces = 0;
+    int need_hi = 0;  // the digit reads the high word
+    u32 pos[ALTOB_MAX_MODES] = {0}, mask[ALTOB_MAX_MODES] = {0}, off[ALTOB_MAX_MODES] = {0};
+    u32 lut[KEY_DIGIT_LUT / 4] = {0};
+};
+
+// (key, payload) pairs on key bits [0, nbits); keys are kw u64 words (lo[], hi[]).
 altob_status radix_sort_pairs(u64* klo, u64* khi, u32* pay, u64* klo_alt,
                               u64* khi_alt, u32* pay_alt, u64 n, int kw,
                               int nbits, cudaStream_t st, bool* result_in_alt);
+// 32-bit keys; perm[k] becomes the position key k came from.
+altob_status radix_argsort_u32(u32* key, u32* perm, u32* key_alt, u32* perm_alt, u64 n, int nbits, cudaStream_t st,
+                               bool* result_in_alt);
+// Field-layout keys (64 low bits and hi_bytes = 0, 1, 4 or 8 bytes of high
+// bits each) into ALTO order; perm as above.
+altob_status alto_sort(u64* klo, void* khi, u32* perm, u64* klo_alt, void* khi_alt, u32* perm_alt, u64 n, int hi_bytes,
+                       const u128* masks, const Fields& f, int alto_bits, cudaStream_t st, bool* result_in_alt);
 
 }  // namespace altob

@@ -335,7 +335,13 @@ static altob_status run_tiled_vt(altob_tensor* t, int mode, void* const* dU, voi
     if (plannable && pl.vec == 1) {
         u64 rows = 0;
         for (int m = 0; m < t->nmode; ++m) rows += t->dims[m];
-        if (t->nnz >= rows) {
+        // The copies cost a few passes over the factors, the scalar rows a
+        // load per lane and nonzero.  Sweeps of order 3, scalar -> padded:
+        // 45,000 rows, 45,001 nonzeros, rank 25, FP32 139 -> 74 us; 400,000
+        // nonzeros 186 -> 98; 1.5M rows and nonzeros, rank 25 925 -> 678, but
+        // rank 50 1122 -> 1183; 3M nonzeros, rank 50 2022 -> 1708.
+        const u64 elems = rows * (R + 3);
+        if (elems <= (4u << 20) ? 4 * t->nnz >= rows : elems <= (48u << 20) ? t->nnz >= rows : t->nnz >= 2 * rows) {
             bool ran = false;
             ALTOB_TRY((run_padded<FT, VT>(t, mode, dU, dout, R, phi, eps, perm, st, &ran)));
             if (ran) return ALTOB_OK;
@@ -628,22 +634,21 @@ altob_status pi_device(altob_tensor* t, int mode, altob_dtype ft, void* const* d
 constexpr u64 PR_CHUNK = 512;
 constexpr int PR_THREADS = 256;
 
-__global__ void k_mode_idx(KeySrc key, Fields fld, int mode, u64 n, u64* __restrict__ idx, u32* __restrict__ iota)
+__global__ void k_mode_idx(KeySrc key, Fields fld, int mode, u64 n, u32* __restrict__ idx)
 {
     for (u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (u64)gridDim.x * blockDim.x) {
         const u64 lo = key.klo[i], hi = key_hi(key, i);
         idx[i] = field(lo, hi, fld.pos[mode], fld.mask[mode]);
-        iota[i] = (u32)i;
     }
 }
 
 template <typename FT, typename VT>
-__global__ void k_row_meta(const u64* __restrict__ sidx, const u32* __restrict__ perm, const VT* __restrict__ vals,
+__global__ void k_row_meta(const u32* __restrict__ sidx, const u32* __restrict__ perm, const VT* __restrict__ vals,
                            u64 n, u32* __restrict__ rows, FT* __restrict__ svals, u32* __restrict__ inv)
 {
     for (u64 k = (u64)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (u64)gridDim.x * blockDim.x) {
         const u32 p = perm[k];
-        rows[k] = (u32)sidx[k];
+        rows[k] = sidx[k];
         svals[k] = (FT)vals[p];
         inv[p] = (u32)k;
     }
@@ -774,7 +779,7 @@ template <typename FT, typename VT>
 static altob_status mode_order_vt(altob_tensor* t, int mode, u32* rows, FT* svals, u32* inv, cudaStream_t st)
 {
     const u64 n = t->nnz;
-    u64 *mk = nullptr, *mk2 = nullptr;
+    u32 *mk = nullptr, *mk2 = nullptr;
     u32 *p = nullptr, *p2 = nullptr;
     altob_status s = dmalloc_t(&mk, n);
     if (s == ALTOB_OK) s = dmalloc_t(&mk2, n);
@@ -785,10 +790,10 @@ static altob_status mode_order_vt(altob_tensor* t, int mode, u32* rows, FT* sval
     const int grid = (int)std::max<u64>(1, std::min<u64>((n + 255) / 256, (u64)num_sms() * 8));
     bool alt = false;
     if (s == ALTOB_OK) {
-        k_mode_idx<<<grid, 256, 0, st>>>(key_src(t), t->fld, mode, n, mk, p);
+        k_mode_idx<<<grid, 256, 0, st>>>(key_src(t), t->fld, mode, n, mk);
         s = cudaGetLastError() == cudaSuccess ? ALTOB_OK : fail(ALTOB_ERR_CUDA, "mode index launch failed");
     }
-    if (s == ALTOB_OK) s = radix_sort_pairs(mk, nullptr, p, mk2, nullptr, p2, n, 1, bits, st, &alt);
+    if (s == ALTOB_OK) s = radix_argsort_u32(mk, p, mk2, p2, n, bits, st, &alt);
     if (s == ALTOB_OK) {
         k_row_meta<FT, VT><<<grid, 256, 0, st>>>(alt ? mk2 : mk, alt ? p2 : p, (const VT*)t->d_vals, n, rows, svals,
                                                  inv);
