@@ -85,6 +85,7 @@ SIGNATURES = {
     "altob_status_string": (C.c_char_p, [_i]),
     "altob_last_error": (C.c_char_p, []),
     "altob_version": (C.c_char_p, []),
+    "altob_trim_memory": (_i, []),
     "altob_create": (_i, [_i, _u64p, _u64, _u64p, _vp, _i, _i, _i, _vp, C.POINTER(_vp)]),
     "altob_create_device": (_i, [_i, _u64p, _u64, _vp, _vp, _i, _i, _i, _vp, C.POINTER(_vp)]),
     "altob_destroy": (_i, [_vp]),
@@ -598,6 +599,12 @@ def status_of(fn, *args):
         return 0
     except AltobError as e:
         return e.status
+
+
+def trim_memory():
+    """Returns the device memory that the library keeps between calls
+    (altob_trim_memory)."""
+    _check(lib().altob_trim_memory())
 
 
 def version():

@@ -245,6 +245,7 @@ static AprPhi apr_phi_kind(const altob_tensor* t, int R, size_t fsz, int max_inn
     if (max_inner < 2) return PHI_OTF;
     size_t fr = 0, tot = 0;
     if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) return PHI_OTF;
+    fr += pool_unused();
     const double nnz = (double)t->nnz;
     if (nnz * ((double)R * fsz + t->nmode * (8.0 + fsz) + 24.0) <= 0.25 * (double)fr) return PHI_ROWS;
     return nnz * R * fsz <= 0.25 * (double)fr ? PHI_PRE : PHI_OTF;

@@ -33,10 +33,58 @@ static thread_local cudaStream_t g_alloc_stream = 0;
 StreamScope::StreamScope(cudaStream_t s) : prev(g_alloc_stream) { g_alloc_stream = s; }
 StreamScope::~StreamScope() { g_alloc_stream = prev; }
 
+// The library's own stream-ordered pool of the current device.  The default
+// pool hands unused memory back to the system at every synchronisation, which
+// made a build spend 8 ms in its 22 allocations; this one keeps up to 1/32 of
+// the device's memory (5.7 GB of 180) between calls.  Kept memory is returned
+// by altob_trim_memory, and by the driver when another allocation of the
+// process needs it.  nullptr: pools cannot be made here, use the default one.
+static cudaMemPool_t device_pool()
+{
+    static std::mutex mu;
+    static std::vector<std::pair<bool, cudaMemPool_t>> pools;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    std::lock_guard<std::mutex> lk(mu);
+    if (dev >= (int)pools.size()) pools.resize(dev + 1, {false, nullptr});
+    if (!pools[dev].first) {
+        cudaMemPoolProps pr;
+        memset(&pr, 0, sizeof(pr));
+        pr.allocType = cudaMemAllocationTypePinned;
+        pr.location.type = cudaMemLocationTypeDevice;
+        pr.location.id = dev;
+        size_t fr = 0, tot = 0;
+        cudaMemPool_t p = nullptr;
+        if (cudaMemGetInfo(&fr, &tot) == cudaSuccess && cudaMemPoolCreate(&p, &pr) == cudaSuccess) {
+            u64 keep = tot / 32;
+            cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep);
+        } else {
+            cudaGetLastError();
+            p = nullptr;
+        }
+        pools[dev] = {true, p};
+    }
+    return pools[dev].second;
+}
+
+size_t pool_unused()
+{
+    cudaMemPool_t p = device_pool();
+    u64 reserved = 0, used = 0;
+    if (!p || cudaMemPoolGetAttribute(p, cudaMemPoolAttrReservedMemCurrent, &reserved) != cudaSuccess ||
+        cudaMemPoolGetAttribute(p, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return reserved > used ? (size_t)(reserved - used) : 0;
+}
+
 altob_status dmalloc(void** p, size_t bytes)
 {
     *p = nullptr;
-    cudaError_t e = cudaMallocAsync(p, bytes ? bytes : 1, g_alloc_stream);
+    cudaMemPool_t pool = device_pool();
+    cudaError_t e = pool ? cudaMallocFromPoolAsync(p, bytes ? bytes : 1, pool, g_alloc_stream)
+                         : cudaMallocAsync(p, bytes ? bytes : 1, g_alloc_stream);
     if (e != cudaSuccess) {
         cudaGetLastError();
         *p = nullptr;
@@ -868,6 +916,13 @@ const char* altob_status_string(altob_status s)
 const char* altob_last_error(void) { return g_last_error.c_str(); }
 
 const char* altob_version(void) { return "alto_b200 0.1.0 (sm_100a)"; }
+
+altob_status altob_trim_memory(void)
+{
+    cudaMemPool_t p = device_pool();
+    if (p) ALTOB_CUDA(cudaMemPoolTrimTo(p, 0));
+    return ALTOB_OK;
+}
 
 altob_status altob_create(int nmode, const uint64_t* dims, uint64_t nnz, const uint64_t* cidx, const void* vals,
                           altob_dtype val_dtype, int nprtn, int lit_bits, void* stream, altob_tensor** out)

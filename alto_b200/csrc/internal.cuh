@@ -258,6 +258,8 @@ altob_status dmalloc_t(T** p, size_t count)
     return dmalloc(reinterpret_cast<void**>(p), count * sizeof(T) + (count == 0));
 }
 void dfree(void* p);
+// Bytes the library's pool holds on the current device but nothing uses.
+size_t pool_unused();
 
 // Per-tensor scratch: returns a device buffer of at least `bytes`, reused
 // across calls on the same handle.

@@ -100,6 +100,13 @@ ALTOB_API const char* altob_last_error(void);
 /* Library version string. */
 ALTOB_API const char* altob_version(void);
 
+/* No counterpart in the reference.  The library keeps up to 1/32 of the
+ * device's memory between calls instead of handing it back to the system at
+ * every synchronisation; this returns what is unused on the current device
+ * (the driver also takes it back when another allocation of the process needs
+ * it).  Memory still in use by work in flight is not waited for. */
+ALTOB_API altob_status altob_trim_memory(void);
+
 /* ---- tensor build ------------------------------------------------------
  * Replaces create_alto<LIT>(SparseTensor*, AltoTensor<LIT>**, int nprtn)
  * (alto.hpp:108-294): packed LSB-first / shortest-first masks (:669-770),

@@ -1,6 +1,7 @@
 """The build's sort over every width of high key words (none, 8, 32 and 64
 bits), around its tile of 4096 keys and on digits that are all equal: the
-encoding is bit-exact against the oracle."""
+encoding is bit-exact against the oracle.  And the library's memory pool
+after a trim."""
 import numpy as np
 import pytest
 
@@ -41,3 +42,15 @@ def test_sort_of_clustered_keys(oracle):
     vals = rng.random(cidx.shape[1])
     at = ab.create_alto(ab.SparseTensor.from_arrays(dims, cidx, vals), 16, 128)
     _check_against(at.dump(), oracle.create(dims, cidx, vals, 16, 128).dump(), dims, vals.shape[0])
+
+
+def test_trim_returns_unused_memory():
+    torch = pytest.importorskip("torch")
+    cidx, v = synth.uniform_coo_torch((3000, 2000, 1000), 4_000_000, 1, "cuda")
+    at = ab.create_alto_device(3, (3000, 2000, 1000), 4_000_000, cidx, v, 16, 0)
+    at.destroy()
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    ab.trim_memory()
+    # the build's buffers (at least keys, payloads and values of 4M nonzeros) were kept and came back
+    assert torch.cuda.mem_get_info()[0] >= before + 4_000_000 * 20
