@@ -21,10 +21,14 @@
 namespace altob {
 
 // |min(B, 1 - Phi)| max-reduced (apr.hpp:1210-1216); with `mult`, also
-// B *= Phi (apr.hpp:1226-1231) in the same pass.
+// B *= Phi (apr.hpp:1226-1231) in the same pass.  stop (if given): nothing is
+// done once it is set.
 template <typename FT>
-__global__ void k_kkt(FT* __restrict__ B, const FT* __restrict__ Phi, u64 n, double* __restrict__ kkt, int mult)
+__global__ void __launch_bounds__(256) k_kkt(FT* __restrict__ B, const FT* __restrict__ Phi, u64 n,
+                                             double* __restrict__ kkt, int mult, const int* __restrict__ stop)
 {
+    if (stop && *stop) return;
+    __shared__ double red[8];
     double m = 0.0;
     for (u64 e = (u64)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (u64)gridDim.x * blockDim.x) {
         const double b = (double)B[e], p = (double)Phi[e];
@@ -32,8 +36,12 @@ __global__ void k_kkt(FT* __restrict__ B, const FT* __restrict__ Phi, u64 n, dou
         if (mult) B[e] = (FT)(b * p);
     }
     for (int o = 16; o; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if ((threadIdx.x & 31) == 0)
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; ++w) m = fmax(m, red[w]);
         atomicMax(reinterpret_cast<unsigned long long*>(kkt), (unsigned long long)__double_as_longlong(m));
+    }
 }
 
 template <typename FT>
@@ -41,6 +49,25 @@ __global__ void k_mult(FT* __restrict__ B, const FT* __restrict__ Phi, u64 n)
 {
     for (u64 e = (u64)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (u64)gridDim.x * blockDim.x)
         B[e] = (FT)((double)B[e] * (double)Phi[e]);
+}
+
+// The end of an inner round without the host: stops the mode's rounds when
+// the violation is below eps (every block reads the same value; one of them
+// sets the flag that later launches read), else B *= Phi, and Phi is zeroed
+// for the next round.
+template <typename FT>
+__global__ void __launch_bounds__(256) k_round_end(FT* __restrict__ B, FT* __restrict__ Phi, u64 n,
+                                                   const double* __restrict__ kkt, double eps, int zero, int* stop)
+{
+    if (*(volatile int*)stop) return;
+    if (*kkt < eps) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) *(volatile int*)stop = 1;
+        return;
+    }
+    for (u64 e = (u64)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (u64)gridDim.x * blockDim.x) {
+        B[e] = (FT)((double)B[e] * (double)Phi[e]);
+        if (zero) Phi[e] = FT(0);
+    }
 }
 
 // Kappa fix (apr.hpp:1176-1189).
@@ -202,7 +229,7 @@ static altob_status loglik_sum(const altob_tensor* t, FT** U, int R, double eps,
 }
 
 struct AprScratch {
-    double *lam, *colacc, *llacc, *kkt, *G, *inner, *fit, *normAT;
+    double *lam, *colacc, *llacc, *rounds, *kkt, *G, *inner, *fit, *normAT;
     int* info;
 };
 
@@ -251,6 +278,28 @@ static AprPhi apr_phi_kind(const altob_tensor* t, int R, size_t fsz, int max_inn
     return nnz * R * fsz <= 0.25 * (double)fr ? PHI_PRE : PHI_OTF;
 }
 
+// Rounds queued between two reads of the stop flag.
+constexpr int APR_GROUP = 2;
+
+// Two pinned words and events for reading a device flag behind the queue.
+struct PollFlag {
+    volatile int* h = nullptr;
+    cudaEvent_t ev[2] = {nullptr, nullptr};
+    altob_status init()
+    {
+        static thread_local int* word = nullptr;  // kept: eight bytes per host thread that ever solved
+        if (!word) ALTOB_CUDA(cudaHostAlloc((void**)&word, 2 * sizeof(int), cudaHostAllocPortable));
+        h = word;
+        for (int k = 0; k < 2; ++k) ALTOB_CUDA(cudaEventCreateWithFlags(&ev[k], cudaEventDisableTiming));
+        return ALTOB_OK;
+    }
+    ~PollFlag()
+    {
+        for (int k = 0; k < 2; ++k)
+            if (ev[k]) cudaEventDestroy(ev[k]);
+    }
+};
+
 template <typename FT>
 static altob_status cp_apr_impl(altob_tensor* t, FT** U, FT* lam_io, int R, int max_iters, int max_inner,
                                 double eps, double eps_div_zero, double kappa_tol, double kappa, int dobench,
@@ -264,7 +313,7 @@ static altob_status cp_apr_impl(altob_tensor* t, FT** U, FT* lam_io, int R, int 
         phi_off[n] = phi_elems;
         phi_elems += (t->dims[n] * R + 63) & ~(size_t)63;
     }
-    size_t nd = 5 * (size_t)R + (size_t)N * R * R + 16;
+    size_t nd = 5 * (size_t)R + (size_t)N * R * R + (size_t)N * (max_inner + 1) + 16;
     size_t bytes = nd * sizeof(double) + 256 + phi_elems * sizeof(FT) + 256;
     void* base = nullptr;
     ALTOB_TRY(tensor_scratch(t, bytes, &base));
@@ -284,6 +333,8 @@ static altob_status cp_apr_impl(altob_tensor* t, FT** U, FT* lam_io, int R, int 
     s.normAT = d++;
     s.llacc = d;
     d += R + 2;
+    s.rounds = d;
+    d += (size_t)N * (max_inner + 1);
     s.info = (int*)d;
     d += 2;
     FT* phi_base = (FT*)(((uintptr_t)d + 255) & ~(uintptr_t)255);
@@ -356,6 +407,12 @@ static altob_status cp_apr_impl(altob_tensor* t, FT** U, FT* lam_io, int R, int 
         }
         pi_free.p = pi;
     }
+    // rounds without the host in between: the row-ordered stream through the
+    // register-staged kernel (the opt-in bulk-copy kernel takes no stop flag)
+    const bool queued = rows && !env_int("ALTOB_PHI_TMA", 0);
+    PollFlag poll;
+    if (queued) ALTOB_TRY(poll.init());
+    std::vector<double> hrounds((size_t)N * (max_inner + 1));
     int iter;
     for (iter = 0; iter < max_iters; ++iter) {
         bool converged = false;
@@ -371,6 +428,34 @@ static altob_status cp_apr_impl(altob_tensor* t, FT** U, FT* lam_io, int R, int 
             ALTOB_TRY(mul_cols<FT>(B, t->dims[n], R, s.lam, st));
             const u32* inv_n = rows ? inv + (size_t)n * nnzp : nullptr;
             if (pi) ALTOB_TRY(pi_device(t, n, ft, (void* const*)U, (u64)R, pi, st, inv_n));
+            if (queued) {
+                // every round of the mode is queued without waiting for its
+                // violation: the rounds after the one that meets eps return at
+                // once.  The stop flag is polled one group of rounds behind,
+                // so the device never waits for the host and few empty rounds
+                // are queued.
+                double* kk = s.rounds + (size_t)n * (max_inner + 1);
+                int* stop = (int*)(kk + max_inner);
+                const double stop_eps = dobench ? -1.0 : eps;  // bench mode: all rounds
+                ALTOB_CUDA(cudaMemsetAsync(kk, 0, (size_t)(max_inner + 1) * sizeof(double), st));
+                ALTOB_CUDA(cudaMemsetAsync(Phi[n], 0, sz * sizeof(FT), st));
+                int group = 0;
+                for (int r = 0; r < max_inner; ++r) {
+                    ALTOB_TRY(phi_rows_device(t, n, ft, pi, rows + (size_t)n * nnzp, svals + (size_t)n * nnzp, B, (u64)R,
+                                              eps_div_zero, Phi[n], st, true, stop));
+                    k_kkt<FT><<<ew_grid(sz), 256, 0, st>>>(B, Phi[n], sz, kk + r, 0, stop);
+                    k_round_end<FT><<<ew_grid(sz), 256, 0, st>>>(B, Phi[n], sz, kk + r, stop_eps, r + 1 < max_inner, stop);
+                    ALTOB_LAUNCH_CHECK();
+                    if (dobench || r + 1 == max_inner || (r + 1) % APR_GROUP) continue;
+                    ALTOB_CUDA(cudaMemcpyAsync((int*)poll.h + group % 2, stop, sizeof(int), cudaMemcpyDeviceToHost, st));
+                    ALTOB_CUDA(cudaEventRecord(poll.ev[group % 2], st));
+                    if (group > 0) {
+                        ALTOB_CUDA(cudaEventSynchronize(poll.ev[(group - 1) % 2]));
+                        if (poll.h[(group - 1) % 2]) break;
+                    }
+                    ++group;
+                }
+            } else {
             for (int inner = 0; inner < max_inner; ++inner) {
                 ninner[iter]++;
                 if (rows)
@@ -381,11 +466,11 @@ static altob_status cp_apr_impl(altob_tensor* t, FT** U, FT* lam_io, int R, int 
                 if (dobench) {
                     // no early exit: the violation of the last round is what the reference reports
                     ALTOB_CUDA(cudaMemsetAsync(s.kkt + n, 0, sizeof(double), st));
-                    if (sz) k_kkt<FT><<<ew_grid(sz), 256, 0, st>>>(B, Phi[n], sz, s.kkt + n, 1);
+                    if (sz) k_kkt<FT><<<ew_grid(sz), 256, 0, st>>>(B, Phi[n], sz, s.kkt + n, 1, nullptr);
                     ALTOB_LAUNCH_CHECK();
                 } else {
                     ALTOB_CUDA(cudaMemsetAsync(s.kkt + n, 0, sizeof(double), st));
-                    if (sz) k_kkt<FT><<<ew_grid(sz), 256, 0, st>>>(B, Phi[n], sz, s.kkt + n, 0);
+                    if (sz) k_kkt<FT><<<ew_grid(sz), 256, 0, st>>>(B, Phi[n], sz, s.kkt + n, 0, nullptr);
                     ALTOB_LAUNCH_CHECK();
                     double kv = 0.0;
                     ALTOB_CUDA(cudaMemcpyAsync(&kv, s.kkt + n, sizeof(double), cudaMemcpyDeviceToHost, st));
@@ -396,11 +481,24 @@ static altob_status cp_apr_impl(altob_tensor* t, FT** U, FT* lam_io, int R, int 
                     ALTOB_LAUNCH_CHECK();
                 }
             }
+            }
             // KruskalModelNormalizeMode (src/kruskal_model.cpp:178-222)
             ALTOB_TRY(colsum_abs<FT>(B, t->dims[n], R, s.colacc, st));
             ALTOB_TRY(div_cols<FT>(B, t->dims[n], R, s.colacc, s.lam, true, st));
         }
-        if (dobench) {
+        if (queued) {
+            // the violations of every round and mode tell which round was the last
+            ALTOB_CUDA(cudaMemcpyAsync(hrounds.data(), s.rounds, hrounds.size() * sizeof(double), cudaMemcpyDeviceToHost,
+                                       st));
+            ALTOB_CUDA(cudaStreamSynchronize(st));
+            for (int n = 0; n < N; ++n) {
+                const double* kk = hrounds.data() + (size_t)n * (max_inner + 1);
+                int r = 0;
+                while (r + 1 < max_inner && (dobench || !(kk[r] < eps))) ++r;
+                ninner[iter] += r + 1;
+                kmode[n] = kk[r];
+            }
+        } else if (dobench) {
             ALTOB_CUDA(cudaMemcpyAsync(kmode.data(), s.kkt, N * sizeof(double), cudaMemcpyDeviceToHost, st));
             ALTOB_CUDA(cudaStreamSynchronize(st));
         }

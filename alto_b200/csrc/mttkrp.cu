@@ -626,12 +626,11 @@ altob_status pi_device(altob_tensor* t, int mode, altob_dtype ft, void* const* d
 // sequential rows: Phi[r] = sum over the run of row r of
 // (v / max(B[r] . pi, eps)) pi, the products and the dot product formed as in
 // the tiled Phi (apr.hpp:383-848 computes the same sums per row).  A warp
-// takes PR_CHUNK consecutive stream positions; each lane group keeps the
+// takes one range of consecutive stream positions; each lane group keeps the
 // running sum of its current row in registers and adds it to Phi with one
 // vector atomic when the row changes (rows change rarely: the runs of a
 // mode are nnz / dims long on average).
 
-constexpr u64 PR_CHUNK = 512;
 constexpr int PR_THREADS = 256;
 
 __global__ void k_mode_idx(KeySrc key, Fields fld, int mode, u64 n, u32* __restrict__ idx)
@@ -654,67 +653,80 @@ __global__ void k_row_meta(const u32* __restrict__ sidx, const u32* __restrict__
     }
 }
 
-// UN nonzeros of a lane group (stream positions k, k + G, ...; rw = ~0 past k1)
+// UN nonzeros of a lane group (stream positions k, k + G, ...; rw = ~0 past
+// k1).  The target rows are read one step ahead of the rest, so the B rows are
+// fetched together with the Khatri-Rao rows: a lane group that meets a new
+// target row finds its B row there instead of waiting for it (the B rows of
+// neighbouring positions are the same lines, an L1 hit).
+template <int UN, int G>
+__device__ __forceinline__ void row_index(const u32* __restrict__ rows, u64 k, u64 k1, u32* rw)
+{
+#pragma unroll
+    for (int u = 0; u < UN; ++u) rw[u] = k + (u64)u * G < k1 ? __ldcs(rows + k + (u64)u * G) : 0xffffffffu;
+}
+
 template <typename FT, int VEC, int LPN, int CH, int UN>
 struct RowStep {
     u32 rw[UN];
-    FT v[UN], x[UN][CH][VEC];
-    __device__ __forceinline__ void load(const FT* __restrict__ Pi, const u32* __restrict__ rows,
-                                         const FT* __restrict__ vals, u64 k, u64 k1, int R, int sub)
+    FT v[UN], x[UN][CH][VEC], b[UN][CH][VEC];
+    __device__ __forceinline__ void load(const FT* __restrict__ Pi, const FT* __restrict__ vals,
+                                         const FT* __restrict__ B, u64 k, const u32* idx, int R, int sub)
     {
         constexpr int G = 32 / LPN;
 #pragma unroll
         for (int u = 0; u < UN; ++u) {
             const u64 ku = k + (u64)u * G;
-            const bool ok = ku < k1;
-            rw[u] = ok ? __ldcs(rows + ku) : 0xffffffffu;
+            rw[u] = idx[u];
+            const bool ok = idx[u] != 0xffffffffu;
             v[u] = ok ? __ldcs(vals + ku) : FT(0);
 #pragma unroll
             for (int ch = 0; ch < CH; ++ch) {
                 const int r0 = ch * LPN * VEC + sub * VEC;
-                if (ok && r0 < R) vload_stream<FT, VEC>(Pi + ku * R + r0, x[u][ch]);
-                else
+                if (ok && r0 < R) {
+                    vload_stream<FT, VEC>(Pi + ku * R + r0, x[u][ch]);
+                    vload<FT, VEC>(B + (size_t)idx[u] * R + r0, b[u][ch]);
+                } else {
 #pragma unroll
-                    for (int e = 0; e < VEC; ++e) x[u][ch][e] = FT(0);
+                    for (int e = 0; e < VEC; ++e) x[u][ch][e] = b[u][ch][e] = FT(0);
+                }
             }
         }
     }
 };
 
 // Adds the step's nonzeros to the lane group's run; a row change flushes the
-// run with one vector atomic per lane and reloads the cached B row.
+// run with one vector atomic per lane.
 template <typename FT, int VEC, int LPN, int CH, int UN>
-__device__ __forceinline__ void row_step(const RowStep<FT, VEC, LPN, CH, UN>& s, const FT* __restrict__ B,
-                                         FT* __restrict__ Phi, int R, int sub, unsigned gmask, FT eps, u32& cur,
-                                         FT (*acc)[VEC], FT (*bc)[VEC])
+__device__ __forceinline__ void row_step(const RowStep<FT, VEC, LPN, CH, UN>& s, FT* __restrict__ Phi, int R, int sub,
+                                         unsigned gmask, FT eps, u32& cur, FT (*acc)[VEC])
 {
+    FT dot[UN];
+#pragma unroll
+    for (int u = 0; u < UN; ++u) {
+        dot[u] = FT(0);
+#pragma unroll
+        for (int ch = 0; ch < CH; ++ch)
+#pragma unroll
+            for (int e = 0; e < VEC; ++e) dot[u] += s.b[u][ch][e] * s.x[u][ch][e];
+    }
+#pragma unroll
+    for (int o = LPN / 2; o > 0; o >>= 1)
+#pragma unroll
+        for (int u = 0; u < UN; ++u) dot[u] += __shfl_xor_sync(gmask, dot[u], o, LPN);
 #pragma unroll
     for (int u = 0; u < UN; ++u) {
         if (s.rw[u] == 0xffffffffu) break;  // past the chunk (uniform in the group)
+        const FT sc = s.v[u] / (dot[u] > eps ? dot[u] : eps);
         if (s.rw[u] != cur) {
 #pragma unroll
             for (int ch = 0; ch < CH; ++ch) {
                 const int r0 = ch * LPN * VEC + sub * VEC;
-                if (r0 < R) {
-                    if (cur != 0xffffffffu) gred<FT, VEC>(Phi + (size_t)cur * R + r0, acc[ch]);
-                    vload<FT, VEC>(B + (size_t)s.rw[u] * R + r0, bc[ch]);
-                }
+                if (r0 < R && cur != 0xffffffffu) gred<FT, VEC>(Phi + (size_t)cur * R + r0, acc[ch]);
 #pragma unroll
                 for (int e = 0; e < VEC; ++e) acc[ch][e] = FT(0);
             }
             cur = s.rw[u];
         }
-        FT dot = FT(0);
-#pragma unroll
-        for (int ch = 0; ch < CH; ++ch) {
-            const int r0 = ch * LPN * VEC + sub * VEC;
-            if (r0 < R)
-#pragma unroll
-                for (int e = 0; e < VEC; ++e) dot += bc[ch][e] * s.x[u][ch][e];
-        }
-#pragma unroll
-        for (int o = LPN / 2; o > 0; o >>= 1) dot += __shfl_xor_sync(gmask, dot, o, LPN);
-        const FT sc = s.v[u] / (dot > eps ? dot : eps);
 #pragma unroll
         for (int ch = 0; ch < CH; ++ch)
 #pragma unroll
@@ -722,48 +734,59 @@ __device__ __forceinline__ void row_step(const RowStep<FT, VEC, LPN, CH, UN>& s,
     }
 }
 
-// Resident blocks per SM the register budget is set for: while a lane holds
-// at most 16 bytes of a stream row, four (64 registers) in FP32 and three in
-// FP64; else two.
+// Steps per register buffer and resident blocks per SM: while a lane holds at
+// most 16 bytes of a stream row, four steps (FP32) or three (FP64) at two
+// blocks, else two steps at two blocks.  Bytes in flight are what the pass
+// needs, not warps: 4.7M nonzeros at rank 16 take 97 us a pass with two steps
+// at four blocks and the B row fetched when the row changes, 70 with two at
+// three blocks and the B rows fetched ahead, 65 with four at two (5.3 TB/s);
+// FP64 207, 172 and, with three steps at two blocks, 152 (four: 180).
 template <typename FT, int VEC, int CH>
-constexpr int pr_min_blocks()
+constexpr int pr_steps()
 {
     return CH * VEC * (int)sizeof(FT) <= 16 ? (sizeof(FT) == 4 ? 4 : 3) : 2;
 }
+constexpr int PR_BLOCKS = 2;
 
 // Two register buffers of UN steps: the loads of the next buffer are issued
 // before the current one is reduced, so a warp keeps 2 x UN x G stream rows
-// in flight.
+// in flight.  stop (if given): the pass does nothing once it is set.
 template <typename FT, int VEC, int LPN, int CH>
-__global__ void __launch_bounds__(PR_THREADS, pr_min_blocks<FT, VEC, CH>()) k_phi_rows(const FT* __restrict__ Pi, const u32* __restrict__ rows,
-                                                         const FT* __restrict__ vals, const FT* __restrict__ B,
-                                                         FT* __restrict__ Phi, u64 nnz, int R, FT eps)
+__global__ void __launch_bounds__(PR_THREADS, PR_BLOCKS)
+    k_phi_rows(const FT* __restrict__ Pi, const u32* __restrict__ rows, const FT* __restrict__ vals,
+               const FT* __restrict__ B, FT* __restrict__ Phi, u64 nnz, int R, FT eps, u64 chunk,
+               const int* __restrict__ stop)
 {
     constexpr int G = 32 / LPN;  // nonzeros per warp step
-    constexpr int UN = 2;
+    constexpr int UN = pr_steps<FT, VEC, CH>();
     constexpr u64 S = (u64)G * UN;
+    if (stop && *stop) return;
     const int lane = threadIdx.x & 31, grp = lane / LPN, sub = lane % LPN;
     const unsigned gmask = LPN == 32 ? 0xffffffffu : (((1u << LPN) - 1u) << (grp * LPN));
-    const u64 nchunks = (nnz + PR_CHUNK - 1) / PR_CHUNK;
     const u64 nw = ((u64)gridDim.x * blockDim.x) >> 5;
-    for (u64 c = ((u64)blockIdx.x * blockDim.x + threadIdx.x) >> 5; c < nchunks; c += nw) {
-        const u64 k1 = min(nnz, (c + 1) * PR_CHUNK);
+    for (u64 c = ((u64)blockIdx.x * blockDim.x + threadIdx.x) >> 5; c * chunk < nnz; c += nw) {
+        const u64 k1 = min(nnz, (c + 1) * chunk);
         u32 cur = 0xffffffffu;
-        FT acc[CH][VEC], bc[CH][VEC];
+        FT acc[CH][VEC];
 #pragma unroll
         for (int ch = 0; ch < CH; ++ch)
 #pragma unroll
-            for (int e = 0; e < VEC; ++e) acc[ch][e] = bc[ch][e] = FT(0);
+            for (int e = 0; e < VEC; ++e) acc[ch][e] = FT(0);
         RowStep<FT, VEC, LPN, CH, UN> a, b;
-        u64 k = c * PR_CHUNK + grp;
-        a.load(Pi, rows, vals, k, k1, R, sub);
+        u32 idx[UN];
+        u64 k = c * chunk + grp;
+        row_index<UN, G>(rows, k, k1, idx);
+        a.load(Pi, vals, B, k, idx, R, sub);
+        row_index<UN, G>(rows, k + S, k1, idx);
         while (k < k1) {
-            b.load(Pi, rows, vals, k + S, k1, R, sub);
-            row_step(a, B, Phi, R, sub, gmask, eps, cur, acc, bc);
+            b.load(Pi, vals, B, k + S, idx, R, sub);
+            row_index<UN, G>(rows, k + 2 * S, k1, idx);
+            row_step(a, Phi, R, sub, gmask, eps, cur, acc);
             k += S;
             if (k >= k1) break;
-            a.load(Pi, rows, vals, k + S, k1, R, sub);
-            row_step(b, B, Phi, R, sub, gmask, eps, cur, acc, bc);
+            a.load(Pi, vals, B, k + S, idx, R, sub);
+            row_index<UN, G>(rows, k + 2 * S, k1, idx);
+            row_step(b, Phi, R, sub, gmask, eps, cur, acc);
             k += S;
         }
         if (cur != 0xffffffffu)
@@ -824,9 +847,9 @@ altob_status mode_order_device(altob_tensor* t, int mode, altob_dtype ft, u32* r
 
 template <typename FT, int VEC>
 static void launch_phi_rows(int lpn, int ch, int grid, const FT* pi, const u32* rows, const FT* vals, const FT* B,
-                            FT* phi, u64 nnz, int R, FT eps, cudaStream_t st)
+                            FT* phi, u64 nnz, int R, FT eps, u64 chunk, const int* stop, cudaStream_t st)
 {
-#define PRK(L, C) k_phi_rows<FT, VEC, L, C><<<grid, PR_THREADS, 0, st>>>(pi, rows, vals, B, phi, nnz, R, eps)
+#define PRK(L, C) k_phi_rows<FT, VEC, L, C><<<grid, PR_THREADS, 0, st>>>(pi, rows, vals, B, phi, nnz, R, eps, chunk, stop)
     if (ch == 4) PRK(32, 4);
     else if (ch == 2) PRK(32, 2);
     else if (lpn == 32) PRK(32, 1);
@@ -912,13 +935,13 @@ static altob_status launch_phi_rows_tma(altob_tensor* t, int lpn, const FT* pi, 
 
 altob_status phi_rows_device(altob_tensor* t, int mode, altob_dtype ft, const void* dpi, const u32* rows,
                              const void* svals, const void* dB, u64 R, double eps, void* dphi, cudaStream_t st,
-                             bool pad4)
+                             bool pad4, const int* stop)
 {
     if (!t || !dpi || !rows || !svals || !dB || !dphi) return fail(ALTOB_ERR_ARG, "NULL argument");
     if (mode < 0 || mode >= t->nmode) return fail(ALTOB_ERR_ARG, "mode out of range");
     if (R == 0 || R > 128) return fail(ALTOB_ERR_UNSUPPORTED, "rank must be 1..128");
     const size_t fsz = ft == ALTOB_F64 ? 8 : 4;
-    ALTOB_CUDA(cudaMemsetAsync(dphi, 0, t->dims[mode] * R * fsz, st));
+    if (!stop) ALTOB_CUDA(cudaMemsetAsync(dphi, 0, t->dims[mode] * R * fsz, st));
     if (t->nnz == 0) return ALTOB_OK;
     const int V = (int)(16 / fsz);
     const bool vec = R % V == 0 && ptr_aligned16(dpi) && ptr_aligned16(dB) && ptr_aligned16(dphi);
@@ -926,14 +949,18 @@ altob_status phi_rows_device(altob_tensor* t, int mode, altob_dtype ft, const vo
     int lpn = 1;
     while (lpn < 32 && (u64)lpn * ve < R) lpn <<= 1;
     const int ch = (int)((R + (u64)lpn * ve - 1) / ((u64)lpn * ve));  // 1, 2 or 4 (only with 32 lanes)
-    const u64 nchunks = (t->nnz + PR_CHUNK - 1) / PR_CHUNK;
-    const int per_sm = ch * ve * (int)fsz <= 16 ? (fsz == 4 ? 4 : 3) : 2;  // pr_min_blocks: one wave
-    const int grid = (int)std::max<u64>(1, std::min<u64>((nchunks + 7) / 8, (u64)num_sms() * per_sm));
+    // every resident warp takes one range of the stream, of at least 32
+    // positions: no partial last wave, and a small tensor still meets every SM
+    // (100,000 nonzeros at rank 32: 31 us a pass in ranges of 512, 6.6 so)
+    const u64 warps = (u64)num_sms() * PR_BLOCKS * (PR_THREADS / 32);
+    const u64 chunk = std::max<u64>(32, ((t->nnz + warps - 1) / warps + 31) / 32 * 32);
+    const u64 nchunks = (t->nnz + chunk - 1) / chunk;
+    const int grid = (int)std::max<u64>(1, std::min<u64>((nchunks + 7) / 8, (u64)num_sms() * PR_BLOCKS));
     const u64 nnz = t->nnz;
     // the stream staged by bulk copies (ALTOB_PHI_TMA=1; measured no faster
     // than the register-staged kernel): one vector chunk per lane, whole
     // 16-byte rows, stream arrays readable to a multiple of 4 past the end
-    if (pad4 && vec && ch == 1 && (R * fsz) % 16 == 0 && env_int("ALTOB_PHI_TMA", 0)) {
+    if (!stop && pad4 && vec && ch == 1 && (R * fsz) % 16 == 0 && env_int("ALTOB_PHI_TMA", 0)) {
         if (ft == ALTOB_F64)
             return launch_phi_rows_tma<double, 2>(t, lpn, (const double*)dpi, rows, (const double*)svals,
                                                   (const double*)dB, (double*)dphi, nnz, (int)R, eps, st);
@@ -942,14 +969,14 @@ altob_status phi_rows_device(altob_tensor* t, int mode, altob_dtype ft, const vo
     }
     if (ft == ALTOB_F64) {
         if (vec) launch_phi_rows<double, 2>(lpn, ch, grid, (const double*)dpi, rows, (const double*)svals,
-                                            (const double*)dB, (double*)dphi, nnz, (int)R, eps, st);
+                                            (const double*)dB, (double*)dphi, nnz, (int)R, eps, chunk, stop, st);
         else launch_phi_rows<double, 1>(lpn, ch, grid, (const double*)dpi, rows, (const double*)svals,
-                                        (const double*)dB, (double*)dphi, nnz, (int)R, eps, st);
+                                        (const double*)dB, (double*)dphi, nnz, (int)R, eps, chunk, stop, st);
     } else {
         if (vec) launch_phi_rows<float, 4>(lpn, ch, grid, (const float*)dpi, rows, (const float*)svals,
-                                           (const float*)dB, (float*)dphi, nnz, (int)R, (float)eps, st);
+                                           (const float*)dB, (float*)dphi, nnz, (int)R, (float)eps, chunk, stop, st);
         else launch_phi_rows<float, 1>(lpn, ch, grid, (const float*)dpi, rows, (const float*)svals,
-                                       (const float*)dB, (float*)dphi, nnz, (int)R, (float)eps, st);
+                                       (const float*)dB, (float*)dphi, nnz, (int)R, (float)eps, chunk, stop, st);
     }
     ALTOB_LAUNCH_CHECK();
     return ALTOB_OK;

@@ -35,9 +35,10 @@ altob_status mode_order_device(altob_tensor* t, int mode, altob_dtype ft, u32* r
                                cudaStream_t st);
 // pad4: rows and svals may be read up to a multiple of 4 elements past the
 // mode's nnz (and start 16-byte aligned), which lets the stream be staged by
-// bulk copies.
+// bulk copies.  stop: a device flag; the caller has zeroed dphi, and the pass
+// does nothing when the flag is set.
 altob_status phi_rows_device(altob_tensor* t, int mode, altob_dtype ft, const void* dpi, const u32* rows,
                              const void* svals, const void* dB, u64 R, double eps, void* dphi, cudaStream_t st,
-                             bool pad4 = false);
+                             bool pad4 = false, const int* stop = nullptr);
 
 }  // namespace altob
