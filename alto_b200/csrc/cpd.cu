@@ -85,17 +85,19 @@ static altob_status cpd_als_impl(altob_tensor* t, FT** U, FT* lam_out, int R, in
     for (int i = 0; i < max_iters; ++i) {
         const NormKind nk = i == 0 ? NORM_2 : NORM_MAX;
         for (int j = 0; j < N; ++j) {
-            ALTOB_TRY(mttkrp_device(t, j, ft, (void* const*)U, (u64)R, 0, ALTOB_ALGO_AUTO, st));
+            // (after the first mode of a fused iteration the output is clear already)
+            ALTOB_TRY(mttkrp_device(t, j, ft, (void* const*)U, (u64)R, fused && j > 0, ALTOB_ALGO_AUTO, st));
             // a shard's partial MTTKRP summed over the GPUs; the dense update
             // below then runs on identical data on every GPU
             ALTOB_TRY(red(U[j], t->dims[j] * (u64)R, ft, ALTOB_REDUCE_SUM, st));
             if (fused) {
                 double* Gj = s.G + (size_t)j * R * R;
                 double* inner = j == N - 1 ? s.inner : nullptr;
-                ALTOB_TRY(solve_setup(s.G, N, j, R, s.W, s.info, st));
+                ALTOB_TRY(solve_setup(s.G, N, j, R, s.W, s.info, st, s.colacc, nk, Gj, inner));
                 ALTOB_TRY(apply_gram<FT>(U[j], t->dims[j], R, s.W, nk, s.colacc, Gj, inner, st));
-                ALTOB_TRY(lambda_finish(s.colacc, R, nk, s.lam, Gj, inner, st));
-                ALTOB_TRY(normalize_cols<FT>(U[j], t->dims[j], R, s.lam, st));
+                ALTOB_TRY(finish_cols<FT>(U[j], t->dims[j], R, s.colacc, nk, s.lam, Gj, inner,
+                                          j + 1 < N ? U[j + 1] : nullptr,
+                                          j + 1 < N ? t->dims[j + 1] * (u64)R * sizeof(FT) : 0, st));
                 continue;
             }
             if (j == N - 1)

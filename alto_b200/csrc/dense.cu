@@ -32,7 +32,8 @@ altob_status gram(const FT* U, u64 I, int R, double* G, const double* div, FT* U
 // Otherwise W = V^+ from a cyclic Jacobi eigendecomposition (eigenvalues
 // below R * eps * max|lambda| dropped).  info[0] += 1 on every fallback.
 
-altob_status solve_setup(const double* G, int nmode, int target, int R, double* W, int* info, cudaStream_t st)
+altob_status solve_setup(const double* G, int nmode, int target, int R, double* W, int* info, cudaStream_t st,
+                         double* colacc, NormKind nk, double* Gj, double* inner)
 {
     if (R > SOLVE_MAX_RANK) return fail(ALTOB_ERR_UNSUPPORTED, "rank above 112 in the R x R solve");
     size_t smem = (size_t)2 * R * R * sizeof(double);
@@ -43,7 +44,8 @@ altob_status solve_setup(const double* G, int nmode, int target, int R, double* 
         while (cur < smem && !configured.compare_exchange_weak(cur, smem)) {
         }
     }
-    k_solve_setup<<<1, DN_THREADS, smem, st>>>(G, nmode, target, R, W, info);
+    k_solve_setup<<<1, DN_THREADS, smem, st>>>(G, nmode, target, R, W, info, colacc, nk == NORM_MAX ? 1.0 : 0.0, Gj,
+                                               inner);
     ALTOB_LAUNCH_CHECK();
     return ALTOB_OK;
 }
@@ -118,10 +120,6 @@ altob_status apply_gram(FT* U, u64 I, int R, const double* W, NormKind nk, doubl
                         cudaStream_t st)
 {
     if (R > APPLY_GRAM_MAX_RANK) return fail(ALTOB_ERR_UNSUPPORTED, "rank above 64 in the fused row update");
-    if (nk == NORM_2) ALTOB_CUDA(cudaMemsetAsync(colacc, 0, (size_t)R * sizeof(double), st));
-    else if (nk == NORM_MAX) ALTOB_TRY(vec_fill(colacc, R, 1.0, st));
-    ALTOB_CUDA(cudaMemsetAsync(G, 0, (size_t)R * R * sizeof(double), st));
-    if (inner) ALTOB_CUDA(cudaMemsetAsync(inner, 0, (size_t)R * sizeof(double), st));
     if (I == 0) return ALTOB_OK;
     switch ((R + 7) / 8) {
     case 1: return launch_apply_gram<FT, 1>(U, I, R, W, nk, colacc, G, inner, st);
@@ -135,24 +133,20 @@ altob_status apply_gram(FT* U, u64 I, int R, const double* W, NormKind nk, doubl
     }
 }
 
-altob_status lambda_finish(const double* colacc, int R, NormKind nk, double* lam, double* G, double* inner,
-                           cudaStream_t st)
-{
-    k_lambda_finish<<<1, DN_THREADS, 0, st>>>(colacc, R, (int)nk, lam, G, inner);
-    ALTOB_LAUNCH_CHECK();
-    return ALTOB_OK;
-}
-
 template <typename FT>
-altob_status normalize_cols(FT* U, u64 I, int R, const double* lam, cudaStream_t st)
+altob_status finish_cols(FT* U, u64 I, int R, const double* colacc, NormKind nk, double* lam, double* G, double* inner,
+                         void* zero, u64 nzero, cudaStream_t st)
 {
-    if (I == 0) return ALTOB_OK;
     constexpr int V = 16 / sizeof(FT);
     const bool vec = R % V == 0 && ((uintptr_t)U & 15) == 0;
     const u64 n = I * (u64)R;
     const size_t smem = (size_t)R * sizeof(double);
-    if (vec) k_div_cols<FT, V><<<dn_grid(n / V, DN_THREADS * 4), DN_THREADS, smem, st>>>(U, I, R, lam);
-    else k_div_cols<FT, 1><<<dn_grid(n, DN_THREADS * 4), DN_THREADS, smem, st>>>(U, I, R, lam);
+    if (vec)
+        k_finish_cols<FT, V><<<dn_grid(n / V, DN_THREADS * 4) + 1, DN_THREADS, smem, st>>>(U, I, R, colacc, (int)nk, lam,
+                                                                                          G, inner, (u32*)zero, nzero);
+    else
+        k_finish_cols<FT, 1><<<dn_grid(n, DN_THREADS * 4) + 1, DN_THREADS, smem, st>>>(U, I, R, colacc, (int)nk, lam, G,
+                                                                                      inner, (u32*)zero, nzero);
     ALTOB_LAUNCH_CHECK();
     return ALTOB_OK;
 }
@@ -254,7 +248,8 @@ altob_status value_sumsq(const altob_tensor* t, double* acc, cudaStream_t st)
     template altob_status apply_w<FT>(FT*, u64, int, const double*, NormKind, double*, cudaStream_t);        \
     template altob_status apply_gram<FT>(FT*, u64, int, const double*, NormKind, double*, double*, double*,  \
                                          cudaStream_t);                                                      \
-    template altob_status normalize_cols<FT>(FT*, u64, int, const double*, cudaStream_t);                    \
+    template altob_status finish_cols<FT>(FT*, u64, int, const double*, NormKind, double*, double*, double*,   \
+                                          void*, u64, cudaStream_t);                                                     \
     template altob_status colsum_abs<FT>(const FT*, u64, int, double*, cudaStream_t);                        \
     template altob_status colsum_abs_sum<FT>(const FT*, u64, int, double*, double*, cudaStream_t);           \
     template altob_status div_cols<FT>(FT*, u64, int, const double*, double*, bool, cudaStream_t);           \

@@ -28,20 +28,25 @@ altob_status check_model(const altob_tensor* t, altob_dtype ft, void* const* dU,
 template <typename FT>
 altob_status gram(const FT* U, u64 I, int R, double* G, const double* div, FT* Uout, const FT* M,
                   double* inner, cudaStream_t st);
-altob_status solve_setup(const double* G, int nmode, int target, int R, double* W, int* info, cudaStream_t st);
+// colacc given: also sets up the accumulators of the apply_gram that follows
+// (column statistics for nk, Gj = 0, inner = 0 if given).
+altob_status solve_setup(const double* G, int nmode, int target, int R, double* W, int* info, cudaStream_t st,
+                         double* colacc = nullptr, NormKind nk = NORM_NONE, double* Gj = nullptr,
+                         double* inner = nullptr);
 template <typename FT>
 altob_status apply_w(FT* U, u64 I, int R, const double* W, NormKind nk, double* colacc, cudaStream_t st);
 altob_status lambda_from(const double* colacc, int R, NormKind nk, double* lam, cudaStream_t st);
-// Fused U <- U W with column statistics, G = U^T U and (inner given) the fit's
-// inner product, all before normalisation; lambda_finish then sets lambda,
-// G /= lambda lambda^T, inner /= lambda; normalize_cols divides U by lambda.
+// Fused U <- U W with column statistics, G += U^T U and (inner given) the
+// fit's inner product, all before normalisation, into accumulators that
+// solve_setup has set up; finish_cols then sets lambda, G /= lambda lambda^T,
+// inner /= lambda, divides U by lambda and clears nzero bytes at zero (the
+// output of the next MTTKRP; nullptr, 0: none).
 template <typename FT>
 altob_status apply_gram(FT* U, u64 I, int R, const double* W, NormKind nk, double* colacc, double* G, double* inner,
                         cudaStream_t st);
-altob_status lambda_finish(const double* colacc, int R, NormKind nk, double* lam, double* G, double* inner,
-                           cudaStream_t st);
 template <typename FT>
-altob_status normalize_cols(FT* U, u64 I, int R, const double* lam, cudaStream_t st);
+altob_status finish_cols(FT* U, u64 I, int R, const double* colacc, NormKind nk, double* lam, double* G, double* inner,
+                         void* zero, u64 nzero, cudaStream_t st);
 altob_status fit_from(const double* G, int nmode, int R, const double* lam, const double* inner, double normAT,
                       double* fit, cudaStream_t st);
 template <typename FT>

@@ -208,70 +208,63 @@ __device__ __forceinline__ void solve_body(const double* __restrict__ G, int nmo
     double* A = ssm;          // R x R
     double* B = ssm + R * R;  // R x R
     __shared__ int ok;
-    const int tid = threadIdx.x;
-    for (int e = tid; e < R * R; e += DN_THREADS) {
-        const int a = e / R, b = e - a * R;
-        const int lo = a >= b ? e : b * R + a;  // symmetric from the lower triangle
-        double v = 1.0;
-        for (int m = 0; m < nmode; ++m)
-            if (m != target) v *= G[(size_t)m * R * R + lo];
-        A[e] = v;
-        B[e] = v;
-    }
-    if (tid == 0) ok = 1;
-    __syncthreads();
-    // right-looking Cholesky of A (lower)
-    for (int k = 0; k < R; ++k) {
-        if (tid == 0) {
-            double d = A[k * R + k];
-            if (!(d > 0.0)) ok = 0;
-            else A[k * R + k] = sqrt(d);
-        }
-        __syncthreads();
-        if (!ok) break;
-        const double dk = A[k * R + k];
-        for (int i = k + 1 + tid; i < R; i += DN_THREADS) A[i * R + k] /= dk;
-        __syncthreads();
-        const int n = R - k - 1;
-        for (int e = tid; e < n * n; e += DN_THREADS) {
-            const int i = k + 1 + e / n, j = k + 1 + e % n;
-            if (j <= i) A[i * R + j] -= A[i * R + k] * A[j * R + k];
-        }
-        __syncthreads();
-    }
-    if (ok) {
-        // Linv (lower) into B, column by column
-        for (int c = tid; c < R; c += DN_THREADS) {
-            for (int i = 0; i < R; ++i) B[i * R + c] = 0.0;
-            B[c * R + c] = 1.0 / A[c * R + c];
-            for (int i = c + 1; i < R; ++i) {
-                double s = 0.0;
-                for (int k = c; k < i; ++k) s += A[i * R + k] * B[k * R + c];
-                B[i * R + c] = -s / A[i * R + i];
+    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+    auto load_v = [&] {
+        for (int a = ty; a < R; a += DN_THREADS / 16)
+            for (int b = tx; b < R; b += 16) {
+                const int lo = a >= b ? a * R + b : b * R + a;  // symmetric from the lower triangle
+                double v = 1.0;
+                for (int m = 0; m < nmode; ++m)
+                    if (m != target) v *= G[(size_t)m * R * R + lo];
+                A[a * R + b] = v;
+                B[a * R + b] = a == b ? 1.0 : 0.0;
             }
+        __syncthreads();
+    };
+    load_v();
+    // Right-looking Cholesky of A (lower) with the same row operations on B,
+    // which turn the identity into L^-1: two barriers per column (scale column
+    // k of A and row k of B by the diagonal; update what is below), every
+    // thread taking the square root of the diagonal itself.  The inverse after
+    // the factorisation, one thread per column, was a serial chain of R^2 / 2
+    // steps: 15.6 us at R = 16 with it, 6.6 now.
+    bool posdef = true;
+    for (int k = 0; k < R; ++k) {
+        const double d = A[k * R + k];
+        if (!(d > 0.0)) {
+            posdef = false;
+            break;
+        }
+        const double dk = sqrt(d);
+        for (int e = tid; e < R; e += DN_THREADS) {
+            if (e > k) A[e * R + k] /= dk;
+            else B[k * R + e] /= dk;
         }
         __syncthreads();
-        for (int e = tid; e < R * R; e += DN_THREADS) {
-            const int a = e / R, b = e - a * R;
-            const int k0 = a > b ? a : b;
-            double s = 0.0;
-            for (int k = k0; k < R; ++k) s += B[k * R + a] * B[k * R + b];
-            W[e] = s;
+        for (int i = k + 1 + ty; i < R; i += DN_THREADS / 16) {
+            const double l = A[i * R + k];
+            for (int j = k + 1 + tx; j <= i; j += 16) A[i * R + j] -= l * A[j * R + k];
+            for (int c = tx; c <= k; c += 16) B[i * R + c] -= l * B[k * R + c];
         }
+        __syncthreads();
+    }
+    if (posdef) {
+        for (int a = ty; a < R; a += DN_THREADS / 16)
+            for (int b = tx; b < R; b += 16) {
+                double s = 0.0;
+                for (int k = a > b ? a : b; k < R; ++k) s += B[k * R + a] * B[k * R + b];
+                W[a * R + b] = s;
+            }
         return;
     }
+    __syncthreads();  // every thread has read the failing diagonal
+    load_v();
     // ---- pseudo-inverse fallback: A = V (symmetric), B = eigenvectors.
     // Two-sided Jacobi with the round-robin (tournament) ordering: each step
     // rotates n/2 disjoint index pairs at once (n = R rounded up to even; the
     // extra index is a dummy), n-1 steps make a sweep.  Sweeps stop when the
     // off-diagonal mass is below 1e-26 of the total (eigenvectors to ~1e-13),
     // at most JAC_SWEEPS of them.
-    for (int e = tid; e < R * R; e += DN_THREADS) {
-        const int a = e / R, b = e - a * R;
-        A[e] = a >= b ? B[e] : B[b * R + a];
-    }
-    __syncthreads();
-    for (int e = tid; e < R * R; e += DN_THREADS) B[e] = (e / R == e % R) ? 1.0 : 0.0;
     const int n = (R + 1) & ~1, half = n / 2;
     __shared__ double jc[JAC_MAX_PAIRS], js[JAC_MAX_PAIRS];
     __shared__ int jp[JAC_MAX_PAIRS], jq[JAC_MAX_PAIRS];
@@ -370,9 +363,21 @@ __device__ __forceinline__ void solve_body(const double* __restrict__ G, int nmo
     if (tid == 0) atomicAdd(info, 1);
 }
 
+// colacc (if given): the accumulators of the row update that follows are set
+// up here instead of by launches of their own: column statistics, the target
+// mode's Gram (not read by this solve) and the fit's inner product.
 static __global__ void __launch_bounds__(DN_THREADS) k_solve_setup(const double* __restrict__ G, int nmode, int target,
-                                                            int R, double* __restrict__ W, int* __restrict__ info)
+                                                            int R, double* __restrict__ W, int* __restrict__ info,
+                                                            double* __restrict__ colacc, double colinit,
+                                                            double* __restrict__ Gj, double* __restrict__ inner)
 {
+    if (colacc) {
+        for (int r = threadIdx.x; r < R; r += DN_THREADS) {
+            colacc[r] = colinit;
+            if (inner) inner[r] = 0.0;
+        }
+        for (int e = threadIdx.x; e < R * R; e += DN_THREADS) Gj[e] = 0.0;
+    }
     solve_body(G, nmode, target, R, W, info);
 }
 
@@ -728,21 +733,17 @@ __device__ __forceinline__ void lambda_finish_body(const double* __restrict__ ac
     }
 }
 
-static __global__ void k_lambda_finish(const double* acc, int R, int nk, double* lam, double* G, double* inner)
-{
-    lambda_finish_body(acc, R, nk, lam, G, inner);
-}
-
 // U[:, c] /= lambda[c] (FT storage, FP64 division as in the reference's
 // normalisation); VEC consecutive elements per thread (R % VEC == 0; 16-byte
 // vectors when VEC * sizeof(FT) == 16), the column index carried along the
 // grid-stride loop.
+// root: `lam` holds column statistics whose square roots are the divisors.
 template <typename FT, int VEC>
 __device__ __forceinline__ void div_cols_body(FT* __restrict__ U, u64 I, int R, const double* __restrict__ lam,
-                                              u64 bx, u64 nbx)
+                                              u64 bx, u64 nbx, bool root = false)
 {
     extern __shared__ double dl_[];
-    for (int r = threadIdx.x; r < R; r += blockDim.x) dl_[r] = lam[r];
+    for (int r = threadIdx.x; r < R; r += blockDim.x) dl_[r] = root ? sqrt(lam[r]) : lam[r];
     __syncthreads();
     const u64 nv = I * (u64)R / VEC;
     const u64 stride = nbx * blockDim.x;
@@ -770,11 +771,25 @@ __device__ __forceinline__ void div_cols_body(FT* __restrict__ U, u64 I, int R, 
     }
 }
 
+// The end of a mode's update in one launch: the last block takes lambda from
+// the column statistics and scales the Gram and the inner product
+// (lambda_finish_body), the others divide U by the lambda they compute
+// themselves, and all of them clear `zero` (nzero bytes, a multiple of 4: the
+// output of the MTTKRP that follows).
 template <typename FT, int VEC>
-__global__ void __launch_bounds__(DN_THREADS) k_div_cols(FT* __restrict__ U, u64 I, int R,
-                                                         const double* __restrict__ lam)
+__global__ void __launch_bounds__(DN_THREADS) k_finish_cols(FT* __restrict__ U, u64 I, int R,
+                                                            const double* __restrict__ acc, int nk,
+                                                            double* __restrict__ lam, double* __restrict__ G,
+                                                            double* __restrict__ inner, u32* __restrict__ zero,
+                                                            u64 nzero)
 {
-    div_cols_body<FT, VEC>(U, I, R, lam, blockIdx.x, gridDim.x);
+    const u64 nz = nzero / 4, step = (u64)gridDim.x * blockDim.x, z0 = (u64)blockIdx.x * blockDim.x + threadIdx.x;
+    if (((uintptr_t)zero & 15) == 0 && nz % 4 == 0)
+        for (u64 e = z0; e < nz / 4; e += step) reinterpret_cast<uint4*>(zero)[e] = make_uint4(0, 0, 0, 0);
+    else
+        for (u64 e = z0; e < nz; e += step) zero[e] = 0;
+    if (blockIdx.x == gridDim.x - 1) lambda_finish_body(acc, R, nk, lam, G, inner);
+    else div_cols_body<FT, VEC>(U, I, R, acc, blockIdx.x, gridDim.x - 1, nk == NORM_2);
 }
 
 // Rank classes of the row kernels: (lanes per row, columns per lane) and

@@ -603,7 +603,12 @@ __device__ __forceinline__ void planned_body(const TiledArgs<FT>& a)
 #pragma unroll
         for (int k = 0; k < MM - 1; ++k) Uo[k] = a.U[k < target ? k : k + 1];
         FT* out = WHOLE ? a.hot_acc + (size_t)blockIdx.x * a.whole * R : a.out;
-        planned_runs<FT, MM, LPN, VEC, CH, PSH, PHI, !WHOLE>(a, gs, srec, srecb, Uo, out, p0, pend, R, sub, gmask);
+        if constexpr (!PHI && !WHOLE && CH == 1 && BW == 0) {
+            gs.srec = srec;
+            lean_runs<FT, MM, LPN, VEC, PSH>(a, gs, Uo, p0, pend, R, sub, gmask);
+        } else {
+            planned_runs<FT, MM, LPN, VEC, CH, PSH, PHI, !WHOLE>(a, gs, srec, srecb, Uo, out, p0, pend, R, sub, gmask);
+        }
         if constexpr (NBUF == 1) __syncthreads();  // the records are overwritten next tile
     }
     if (slots) {  // the CTA's sums, once each (read from L2, where the atomics landed)
