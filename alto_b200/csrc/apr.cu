@@ -23,17 +23,25 @@ namespace altob {
 // |min(B, 1 - Phi)| max-reduced (apr.hpp:1210-1216); with `mult`, also
 // B *= Phi (apr.hpp:1226-1231) in the same pass.  stop (if given): nothing is
 // done once it is set.
-template <typename FT>
+template <typename FT, int VEC>
 __global__ void __launch_bounds__(256) k_kkt(FT* __restrict__ B, const FT* __restrict__ Phi, u64 n,
                                              double* __restrict__ kkt, int mult, const int* __restrict__ stop)
 {
+    typedef typename VecT<FT, VEC>::T V;
     if (stop && *stop) return;
     __shared__ double red[8];
     double m = 0.0;
-    for (u64 e = (u64)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (u64)gridDim.x * blockDim.x) {
-        const double b = (double)B[e], p = (double)Phi[e];
-        m = fmax(m, fabs(fmin(b, 1.0 - p)));
-        if (mult) B[e] = (FT)(b * p);
+    for (u64 e = (u64)blockIdx.x * blockDim.x + threadIdx.x; e < n / VEC; e += (u64)gridDim.x * blockDim.x) {
+        V bv = reinterpret_cast<const V*>(B)[e];
+        const V pv = reinterpret_cast<const V*>(Phi)[e];
+        FT* b = reinterpret_cast<FT*>(&bv);
+        const FT* p = reinterpret_cast<const FT*>(&pv);
+#pragma unroll
+        for (int k = 0; k < VEC; ++k) {
+            m = fmax(m, fabs(fmin((double)b[k], 1.0 - (double)p[k])));
+            if (mult) b[k] = (FT)((double)b[k] * (double)p[k]);
+        }
+        if (mult) reinterpret_cast<V*>(B)[e] = bv;
     }
     for (int o = 16; o; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
@@ -55,19 +63,54 @@ __global__ void k_mult(FT* __restrict__ B, const FT* __restrict__ Phi, u64 n)
 // the violation is below eps (every block reads the same value; one of them
 // sets the flag that later launches read), else B *= Phi, and Phi is zeroed
 // for the next round.
-template <typename FT>
+template <typename FT, int VEC>
 __global__ void __launch_bounds__(256) k_round_end(FT* __restrict__ B, FT* __restrict__ Phi, u64 n,
                                                    const double* __restrict__ kkt, double eps, int zero, int* stop)
 {
+    typedef typename VecT<FT, VEC>::T V;
     if (*(volatile int*)stop) return;
     if (*kkt < eps) {
         if (blockIdx.x == 0 && threadIdx.x == 0) *(volatile int*)stop = 1;
         return;
     }
-    for (u64 e = (u64)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (u64)gridDim.x * blockDim.x) {
-        B[e] = (FT)((double)B[e] * (double)Phi[e]);
-        if (zero) Phi[e] = FT(0);
+    for (u64 e = (u64)blockIdx.x * blockDim.x + threadIdx.x; e < n / VEC; e += (u64)gridDim.x * blockDim.x) {
+        V bv = reinterpret_cast<const V*>(B)[e];
+        const V pv = reinterpret_cast<const V*>(Phi)[e];
+        FT* b = reinterpret_cast<FT*>(&bv);
+        const FT* p = reinterpret_cast<const FT*>(&pv);
+#pragma unroll
+        for (int k = 0; k < VEC; ++k) b[k] = (FT)((double)b[k] * (double)p[k]);
+        reinterpret_cast<V*>(B)[e] = bv;
+        if (zero) vstore_zero<FT, VEC>(Phi + e * VEC);
     }
+}
+
+// The two above, in 16-byte pieces where B allows it (Phi is aligned).
+template <typename FT>
+static altob_status launch_kkt(FT* B, const FT* Phi, u64 n, double* kkt, int mult, const int* stop, cudaStream_t st)
+{
+    constexpr int V = 16 / sizeof(FT);
+    const bool vec = ptr_aligned16(B) && n % V == 0;
+    const u64 pieces = vec ? n / V : n;
+    const int g = (int)std::max<u64>(1, std::min<u64>((pieces + 511) / 512, (u64)num_sms() * 8));
+    if (vec) k_kkt<FT, V><<<g, 256, 0, st>>>(B, Phi, n, kkt, mult, stop);
+    else k_kkt<FT, 1><<<g, 256, 0, st>>>(B, Phi, n, kkt, mult, stop);
+    ALTOB_LAUNCH_CHECK();
+    return ALTOB_OK;
+}
+
+template <typename FT>
+static altob_status launch_round_end(FT* B, FT* Phi, u64 n, const double* kkt, double eps, int zero, int* stop,
+                                     cudaStream_t st)
+{
+    constexpr int V = 16 / sizeof(FT);
+    const bool vec = ptr_aligned16(B) && n % V == 0;
+    const u64 pieces = vec ? n / V : n;
+    const int g = (int)std::max<u64>(1, std::min<u64>((pieces + 511) / 512, (u64)num_sms() * 8));
+    if (vec) k_round_end<FT, V><<<g, 256, 0, st>>>(B, Phi, n, kkt, eps, zero, stop);
+    else k_round_end<FT, 1><<<g, 256, 0, st>>>(B, Phi, n, kkt, eps, zero, stop);
+    ALTOB_LAUNCH_CHECK();
+    return ALTOB_OK;
 }
 
 // Kappa fix (apr.hpp:1176-1189).
@@ -443,9 +486,8 @@ static altob_status cp_apr_impl(altob_tensor* t, FT** U, FT* lam_io, int R, int 
                 for (int r = 0; r < max_inner; ++r) {
                     ALTOB_TRY(phi_rows_device(t, n, ft, pi, rows + (size_t)n * nnzp, svals + (size_t)n * nnzp, B, (u64)R,
                                               eps_div_zero, Phi[n], st, true, stop));
-                    k_kkt<FT><<<ew_grid(sz), 256, 0, st>>>(B, Phi[n], sz, kk + r, 0, stop);
-                    k_round_end<FT><<<ew_grid(sz), 256, 0, st>>>(B, Phi[n], sz, kk + r, stop_eps, r + 1 < max_inner, stop);
-                    ALTOB_LAUNCH_CHECK();
+                    ALTOB_TRY(launch_kkt<FT>(B, Phi[n], sz, kk + r, 0, stop, st));
+                    ALTOB_TRY(launch_round_end<FT>(B, Phi[n], sz, kk + r, stop_eps, r + 1 < max_inner, stop, st));
                     if (dobench || r + 1 == max_inner || (r + 1) % APR_GROUP) continue;
                     ALTOB_CUDA(cudaMemcpyAsync((int*)poll.h + group % 2, stop, sizeof(int), cudaMemcpyDeviceToHost, st));
                     ALTOB_CUDA(cudaEventRecord(poll.ev[group % 2], st));
@@ -466,12 +508,10 @@ static altob_status cp_apr_impl(altob_tensor* t, FT** U, FT* lam_io, int R, int 
                 if (dobench) {
                     // no early exit: the violation of the last round is what the reference reports
                     ALTOB_CUDA(cudaMemsetAsync(s.kkt + n, 0, sizeof(double), st));
-                    if (sz) k_kkt<FT><<<ew_grid(sz), 256, 0, st>>>(B, Phi[n], sz, s.kkt + n, 1, nullptr);
-                    ALTOB_LAUNCH_CHECK();
+                    ALTOB_TRY(launch_kkt<FT>(B, Phi[n], sz, s.kkt + n, 1, nullptr, st));
                 } else {
                     ALTOB_CUDA(cudaMemsetAsync(s.kkt + n, 0, sizeof(double), st));
-                    if (sz) k_kkt<FT><<<ew_grid(sz), 256, 0, st>>>(B, Phi[n], sz, s.kkt + n, 0, nullptr);
-                    ALTOB_LAUNCH_CHECK();
+                    ALTOB_TRY(launch_kkt<FT>(B, Phi[n], sz, s.kkt + n, 0, nullptr, st));
                     double kv = 0.0;
                     ALTOB_CUDA(cudaMemcpyAsync(&kv, s.kkt + n, sizeof(double), cudaMemcpyDeviceToHost, st));
                     ALTOB_CUDA(cudaStreamSynchronize(st));

@@ -44,9 +44,8 @@ altob_status solve_setup(const double* G, int nmode, int target, int R, double* 
         while (cur < smem && !configured.compare_exchange_weak(cur, smem)) {
         }
     }
-    k_solve_setup<<<1, DN_THREADS, smem, st>>>(G, nmode, target, R, W, info, colacc, nk == NORM_MAX ? 1.0 : 0.0, Gj,
-                                               inner);
-    ALTOB_LAUNCH_CHECK();
+    ALTOB_CUDA(launch_dependent(colacc && !stream_capturing(st), k_solve_setup, dim3(1), dim3(DN_THREADS), smem, st, G, nmode,
+                                target, R, W, info, colacc, nk == NORM_MAX ? 1.0 : 0.0, Gj, inner));
     return ALTOB_OK;
 }
 
@@ -109,9 +108,8 @@ static altob_status launch_apply_gram(FT* U, u64 I, int R, const double* W, Norm
     const u64 want = (groups + per_block - 1) / per_block;
     const int grid = (int)std::max<u64>(1, std::min<u64>(want, (u64)num_sms() * per_sm.load()));
     const int vec_ok = ((uintptr_t)U & 15) == 0;
-    k_apply_gram<FT, MB><<<grid, AG_THREADS, apply_gram_smem<MB>(), st>>>(U, I, R, W, (int)nk, colacc, G, inner,
-                                                                        vec_ok);
-    ALTOB_LAUNCH_CHECK();
+    ALTOB_CUDA(launch_dependent(!stream_capturing(st), k_apply_gram<FT, MB>, dim3(grid), dim3(AG_THREADS),
+                                apply_gram_smem<MB>(), st, U, I, R, W, (int)nk, colacc, G, inner, vec_ok));
     return ALTOB_OK;
 }
 
@@ -141,13 +139,13 @@ altob_status finish_cols(FT* U, u64 I, int R, const double* colacc, NormKind nk,
     const bool vec = R % V == 0 && ((uintptr_t)U & 15) == 0;
     const u64 n = I * (u64)R;
     const size_t smem = (size_t)R * sizeof(double);
+    const bool dep = !stream_capturing(st);
     if (vec)
-        k_finish_cols<FT, V><<<dn_grid(n / V, DN_THREADS * 4) + 1, DN_THREADS, smem, st>>>(U, I, R, colacc, (int)nk, lam,
-                                                                                          G, inner, (u32*)zero, nzero);
+        ALTOB_CUDA(launch_dependent(dep, k_finish_cols<FT, V>, dim3(dn_grid(n / V, DN_THREADS * 4) + 1), dim3(DN_THREADS), smem,
+                                    st, U, I, R, colacc, (int)nk, lam, G, inner, (u32*)zero, nzero));
     else
-        k_finish_cols<FT, 1><<<dn_grid(n, DN_THREADS * 4) + 1, DN_THREADS, smem, st>>>(U, I, R, colacc, (int)nk, lam, G,
-                                                                                      inner, (u32*)zero, nzero);
-    ALTOB_LAUNCH_CHECK();
+        ALTOB_CUDA(launch_dependent(dep, k_finish_cols<FT, 1>, dim3(dn_grid(n, DN_THREADS * 4) + 1), dim3(DN_THREADS), smem, st,
+                                    U, I, R, colacc, (int)nk, lam, G, inner, (u32*)zero, nzero));
     return ALTOB_OK;
 }
 

@@ -371,6 +371,8 @@ static __global__ void __launch_bounds__(DN_THREADS) k_solve_setup(const double*
                                                             double* __restrict__ colacc, double colinit,
                                                             double* __restrict__ Gj, double* __restrict__ inner)
 {
+    grid_trigger();
+    grid_wait();
     if (colacc) {
         for (int r = threadIdx.x; r < R; r += DN_THREADS) {
             colacc[r] = colinit;
@@ -711,6 +713,8 @@ __global__ void __launch_bounds__(AG_THREADS) k_apply_gram(FT* __restrict__ U, u
                                                            double* __restrict__ colacc, double* __restrict__ G,
                                                            double* __restrict__ inner, int vec_ok)
 {
+    grid_trigger();
+    grid_wait();
     apply_gram_body<FT, MB>(U, I, R, W, nk, colacc, G, inner, vec_ok, blockIdx.x, gridDim.x);
 }
 
@@ -783,6 +787,8 @@ __global__ void __launch_bounds__(DN_THREADS) k_finish_cols(FT* __restrict__ U, 
                                                             double* __restrict__ inner, u32* __restrict__ zero,
                                                             u64 nzero)
 {
+    grid_trigger();
+    grid_wait();
     const u64 nz = nzero / 4, step = (u64)gridDim.x * blockDim.x, z0 = (u64)blockIdx.x * blockDim.x + threadIdx.x;
     if (((uintptr_t)zero & 15) == 0 && nz % 4 == 0)
         for (u64 e = z0; e < nz / 4; e += step) reinterpret_cast<uint4*>(zero)[e] = make_uint4(0, 0, 0, 0);

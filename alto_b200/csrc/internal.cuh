@@ -284,6 +284,44 @@ struct TensorUse {
 
 int num_sms();
 
+// Programmatic dependent launch: a kernel launched by launch_dependent may
+// start while the kernel before it on the stream still runs, and must not
+// touch what that kernel writes (or anything an earlier one may still use)
+// before grid_wait(); grid_wait() returns at once in a kernel launched
+// normally.  grid_trigger() lets the dependent kernel start before this one
+// ends.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+inline cudaError_t launch_dependent_raw(const void* k, dim3 grid, dim3 block, void** args, size_t smem, cudaStream_t st)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelExC(&cfg, k, args);
+}
+
+template <typename T>
+struct SameType {
+    typedef T type;
+};
+// `dependent` false: an ordinary launch.  The arguments convert to the kernel's types.
+template <typename... P>
+cudaError_t launch_dependent(bool dependent, void (*k)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                             typename SameType<P>::type... a)
+{
+    void* args[] = {(void*)&a...};
+    return dependent ? launch_dependent_raw((const void*)k, grid, block, args, smem, st)
+                     : cudaLaunchKernel((const void*)k, grid, block, args, smem, st);
+}
+
 // Integer setting from the environment (dflt when unset or empty).
 inline int env_int(const char* name, int dflt)
 {

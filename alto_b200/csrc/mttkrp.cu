@@ -274,7 +274,7 @@ static unsigned pad_grid(u64 rows, int R)
 
 template <typename FT, typename VT>
 static altob_status run_tiled_vt(altob_tensor* t, int mode, void* const* dU, void* dout, u64 R, bool phi,
-                                 double eps, const u32* perm, bool cache, cudaStream_t st);
+                                 double eps, const u32* perm, bool cache, bool after_clear, cudaStream_t st);
 
 // MTTKRP / Phi on padded copies of the factors; *ran = false when the copies
 // cannot be allocated (the caller then runs the scalar-row kernel).
@@ -313,17 +313,20 @@ static altob_status run_padded(altob_tensor* t, int mode, void* const* dU, void*
     pa.Rp = (int)Rp;
     k_pad_rows<FT><<<dim3(pad_grid(most, (int)Rp), n), 256, 0, st>>>(pa);
     ALTOB_LAUNCH_CHECK();
-    ALTOB_TRY((run_tiled_vt<FT, VT>(t, mode, pU, po, Rp, phi, eps, perm, true, st)));
+    ALTOB_TRY((run_tiled_vt<FT, VT>(t, mode, pU, po, Rp, phi, eps, perm, true, false, st)));
     k_unpad_add<FT><<<pad_grid(t->dims[mode], (int)R), 256, 0, st>>>((FT*)dout, po, t->dims[mode], (int)R, (int)Rp);
     ALTOB_LAUNCH_CHECK();
     *ran = true;
     return ALTOB_OK;
 }
 
+// after_clear: the last launch on the stream is one that this call may overlap
+// (k_clear, or a solver's finish_cols): it writes nothing but factors.
 template <typename FT, typename VT>
 static altob_status run_tiled_vt(altob_tensor* t, int mode, void* const* dU, void* dout, u64 R, bool phi,
-                                 double eps, const u32* perm, bool cache, cudaStream_t st)
+                                 double eps, const u32* perm, bool cache, bool after_clear, cudaStream_t st)
 {
+    const bool had_plan = t->d_plan[mode] != nullptr;
     bool aligned = ptr_aligned16(dout);
     for (int m = 0; m < t->nmode; ++m) aligned = aligned && ptr_aligned16(dU[m]);
     TiledPlan pl;
@@ -402,6 +405,8 @@ static altob_status run_tiled_vt(altob_tensor* t, int mode, void* const* dU, voi
         while ((a.ntiles << (a.split_shift + 1)) <= cap && (ipg >> (a.split_shift + 1)) >= 2) ++a.split_shift;
         const u64 items = a.ntiles << a.split_shift;
         c.grid = dim3((unsigned)std::max<u64>(1, std::min<u64>(items, cap)));
+        // a plan built by this call is not complete before the launch
+        c.dependent = after_clear && (perm || had_plan);
         const u64 per_cta = a.ntiles / c.grid.x;
         // one item per CTA: a hot-row table would pass every run on unchanged;
         // in FP64, where it only saves contended atomics, it repays clearing
@@ -427,11 +432,11 @@ static altob_status run_tiled_vt(altob_tensor* t, int mode, void* const* dU, voi
 
 template <typename FT>
 static altob_status run_tiled(altob_tensor* t, int mode, void* const* dU, void* dout, u64 R, bool phi, double eps,
-                              const u32* perm, bool cache, cudaStream_t st)
+                              const u32* perm, bool cache, bool after_clear, cudaStream_t st)
 {
     const bool f64 = sizeof(FT) == 8;
-    if (t->vdt == ALTOB_U32) return run_tiled_vt<FT, u32>(t, mode, dU, dout, R, phi, eps, perm, cache, st);
-    if ((t->vdt == ALTOB_F64) == f64) return run_tiled_vt<FT, FT>(t, mode, dU, dout, R, phi, eps, perm, cache, st);
+    if (t->vdt == ALTOB_U32) return run_tiled_vt<FT, u32>(t, mode, dU, dout, R, phi, eps, perm, cache, after_clear, st);
+    if ((t->vdt == ALTOB_F64) == f64) return run_tiled_vt<FT, FT>(t, mode, dU, dout, R, phi, eps, perm, cache, after_clear, st);
     return fail(ALTOB_ERR_UNSUPPORTED, "stored value dtype does not match the compute dtype");
 }
 
@@ -471,8 +476,43 @@ altob_algo resolve_algo(const altob_tensor* t, int mode, altob_algo algo)
     return ALTOB_ALGO_ATOMIC;
 }
 
+// Clears an output and lets the kernel after it start meanwhile.
+__global__ void __launch_bounds__(256) k_clear(u32* p, u64 n)
+{
+    grid_trigger();
+    const u64 t = (u64)blockIdx.x * blockDim.x + threadIdx.x, step = (u64)gridDim.x * blockDim.x;
+    if (((uintptr_t)p & 15) == 0) {
+        for (u64 e = t; e < n / 4; e += step) reinterpret_cast<uint4*>(p)[e] = make_uint4(0, 0, 0, 0);
+        if (t < n % 4) p[n / 4 * 4 + t] = 0;
+    } else {
+        for (u64 e = t; e < n; e += step) p[e] = 0;
+    }
+}
+
+// Zeroes an output for the planned kernel that follows; *overlap tells whether
+// that kernel may start meanwhile.  Worth it where the kernel outlasts the
+// host's two launches (about 8 us, 32 MB of gathered rows; below, a memset and
+// an ordinary launch cost the host less: 40,000 nonzeros of order 3 at rank 16,
+// FP64, 28.3 against 31.9 us a sweep) and the output is small against the
+// gathers (1M nonzeros 88 -> 84 us a sweep, 150,001 of order 5 at rank 64 99 ->
+// 90; clearing 614 MB outputs so took 6943 against 6840).
+static altob_status clear_output(const altob_tensor* t, void* p, u64 bytes, u64 R, size_t fsz, bool* overlap,
+                                 cudaStream_t st)
+{
+    *overlap = false;
+    if (t->nnz * (u64)(t->nmode - 1) * R * fsz < (32u << 20) || bytes > (16u << 20) || stream_capturing(st)) {
+        ALTOB_CUDA(cudaMemsetAsync(p, 0, bytes, st));
+        return ALTOB_OK;
+    }
+    const u64 n = bytes / 4;  // factors are whole 4-byte words
+    k_clear<<<(unsigned)std::max<u64>(1, std::min<u64>((n + 4095) / 4096, (u64)num_sms() * 8)), 256, 0, st>>>((u32*)p, n);
+    ALTOB_LAUNCH_CHECK();
+    *overlap = true;
+    return ALTOB_OK;
+}
+
 altob_status mttkrp_device(altob_tensor* t, int mode, altob_dtype ft, void* const* dU, u64 R, int accumulate,
-                           altob_algo algo, cudaStream_t st)
+                           altob_algo algo, cudaStream_t st, bool after_clear)
 {
     if (!t || !dU) return fail(ALTOB_ERR_ARG, "NULL argument");
     if (mode < 0 || mode >= t->nmode) return fail(ALTOB_ERR_ARG, "mode out of range");
@@ -483,7 +523,8 @@ altob_status mttkrp_device(altob_tensor* t, int mode, altob_dtype ft, void* cons
     const size_t fsz = ft == ALTOB_F64 ? 8 : 4;
     ALTOB_TRY(tensor_enter(t, st));
     TensorUse use(t, st);
-    if (!accumulate) ALTOB_CUDA(cudaMemsetAsync(dU[mode], 0, t->dims[mode] * R * fsz, st));
+    after_clear = after_clear && !stream_capturing(st);
+    if (!accumulate) ALTOB_TRY(clear_output(t, dU[mode], t->dims[mode] * R * fsz, R, fsz, &after_clear, st));
     if (t->nnz == 0) return ALTOB_OK;
     algo = resolve_algo(t, mode, algo);
     const u32* perm = nullptr;
@@ -499,8 +540,8 @@ altob_status mttkrp_device(altob_tensor* t, int mode, altob_dtype ft, void* cons
         return ft == ALTOB_F64 ? run_atomic_cr<double>(t, mode, dU, R, st) : run_atomic_cr<float>(t, mode, dU, R, st);
     default: return fail(ALTOB_ERR_ARG, "unknown algorithm");
     }
-    return ft == ALTOB_F64 ? run_tiled<double>(t, mode, dU, dU[mode], R, false, 0.0, perm, cache, st)
-                           : run_tiled<float>(t, mode, dU, dU[mode], R, false, 0.0, perm, cache, st);
+    return ft == ALTOB_F64 ? run_tiled<double>(t, mode, dU, dU[mode], R, false, 0.0, perm, cache, after_clear, st)
+                           : run_tiled<float>(t, mode, dU, dU[mode], R, false, 0.0, perm, cache, after_clear, st);
 }
 
 altob_status phi_device(altob_tensor* t, int mode, altob_dtype ft, void* const* dU, u64 R, double eps,
@@ -512,10 +553,11 @@ altob_status phi_device(altob_tensor* t, int mode, altob_dtype ft, void* const* 
     const size_t fsz = ft == ALTOB_F64 ? 8 : 4;
     ALTOB_TRY(tensor_enter(t, st));
     TensorUse use(t, st);
-    ALTOB_CUDA(cudaMemsetAsync(dphi, 0, t->dims[mode] * R * fsz, st));
+    bool dep = false;
+    ALTOB_TRY(clear_output(t, dphi, t->dims[mode] * R * fsz, R, fsz, &dep, st));
     if (t->nnz == 0) return ALTOB_OK;
-    return ft == ALTOB_F64 ? run_tiled<double>(t, mode, dU, dphi, R, true, eps, nullptr, true, st)
-                           : run_tiled<float>(t, mode, dU, dphi, R, true, eps, nullptr, true, st);
+    return ft == ALTOB_F64 ? run_tiled<double>(t, mode, dU, dphi, R, true, eps, nullptr, true, dep, st)
+                           : run_tiled<float>(t, mode, dU, dphi, R, true, eps, nullptr, true, dep, st);
 }
 
 // ------------------------------------------------- precomputed Phi rows

@@ -14,6 +14,7 @@ struct TiledCfg {
     int grouped = 1;  // 1: k_grouped, 0: k_tiled
     int pre = 0;      // Phi from precomputed Khatri-Rao rows (grouped only)
     int planned = 0;  // batched MTTKRP: tiles with a tile plan
+    int dependent = 0;  // planned kernel: launched as a dependent of the kernel that clears its output
     dim3 grid;
     size_t smem = 0;
 };
@@ -52,7 +53,8 @@ altob_status launch_kernel(K k, std::atomic<size_t>& configured, const void* arg
     }
     if (c.grid.x == 0) return ALTOB_OK;
     void* args[] = {const_cast<void*>(args_ptr)};
-    cudaError_t e = cudaLaunchKernel((const void*)k, c.grid, dim3(MT_THREADS), args, c.smem, st);
+    cudaError_t e = c.dependent ? launch_dependent_raw((const void*)k, c.grid, dim3(MT_THREADS), args, c.smem, st)
+                                : cudaLaunchKernel((const void*)k, c.grid, dim3(MT_THREADS), args, c.smem, st);
     if (e != cudaSuccess) return fail(ALTOB_ERR_CUDA, std::string("MTTKRP launch: ") + cudaGetErrorString(e));
     return ALTOB_OK;
 }

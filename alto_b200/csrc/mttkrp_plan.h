@@ -17,8 +17,10 @@ altob_algo resolve_algo(const altob_tensor* t, int mode, altob_algo algo);
 // The tile plan of `mode` (built on first use; nullptr when plans are off or
 // cannot be allocated).
 const uint16_t* tensor_plan(altob_tensor* t, int mode, cudaStream_t st);
+// after_clear: the last launch on st is finish_cols, which the MTTKRP may
+// overlap up to its first read of a factor.
 altob_status mttkrp_device(altob_tensor* t, int mode, altob_dtype ft, void* const* dU, u64 R, int accumulate,
-                           altob_algo algo, cudaStream_t st);
+                           altob_algo algo, cudaStream_t st, bool after_clear = false);
 altob_status phi_device(altob_tensor* t, int mode, altob_dtype ft, void* const* dU, u64 R, double eps,
                         void* dphi, cudaStream_t st);
 // Khatri-Rao rows of every nonzero for `mode` (nnz x R, ALTO order) and Phi

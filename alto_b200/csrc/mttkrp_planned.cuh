@@ -595,6 +595,10 @@ __device__ __forceinline__ void planned_body(const TiledArgs<FT>& a)
         // with two buffers one barrier per tile: the buffer written next tile
         // was last read before this barrier
         __syncthreads();
+        // up to here only keys, values and the plan were read (and the CTA's
+        // own accumulators written); factors and output may still be in the
+        // hands of the kernel before this one
+        if (it == blockIdx.x) grid_wait();
         // ---- B: runs of equal output rows
         const int ipg = IPG >> ssh;
         const int p0 = grp * IPG + (int)(it & ((1u << ssh) - 1u)) * ipg;
