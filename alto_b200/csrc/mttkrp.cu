@@ -383,8 +383,11 @@ static altob_status run_tiled_vt(altob_tensor* t, int mode, void* const* dU, voi
         // runs of 16 or more nonzeros through the hot-row table: fewer table
         // lookups than at 8 (2.19 -> 2.16 ms per mode on the 100.85M-nonzero
         // Zipf tensor) at the same FP32 error (1.0-1.7e-6 against FP64); below
-        // 8 the lookups cost more than the atomics they save (2: 2.61 ms)
-        a.hot_minrun = 16;
+        // 8 the lookups cost more than the atomics they save (2: 2.61 ms); FP64
+        // adds with one atomic per element, so its line lies lower (28.8M
+        // nonzeros of a Zipf tensor at rank 32: 5.39 ms a sweep at 16, 5.24 at
+        // 8, 5.28 at 4)
+        a.hot_minrun = sizeof(FT) == 8 ? 8 : 16;
         a.hot = env_int("ALTOB_HOT_ROWS", 1) ? hot_slots((int)R, sizeof(FT)) : 0;
         a.tile = PT_TILE;
         a.ntiles = (t->nnz + PT_TILE - 1) / PT_TILE;

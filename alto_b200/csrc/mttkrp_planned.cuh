@@ -198,13 +198,14 @@ __global__ void __launch_bounds__(TILE / TP_IPT) k_tile_plan(KeySrc key, Fields 
 // at 5 on the 100.85M-nonzero Zipf tensor; 3 blocks: 2.53 ms), 4 above rank
 // 64 (32 lanes per nonzero spill at 48 registers).  FP32 orders 4-5 and Phi:
 // 4 (on 18.9M nonzeros of order 4 at rank 16 Phi takes 490 us a mode at 3
-// blocks, 467 at 4, 484 at 5; the order-4 MTTKRP 348, 350, 470).  FP64 order
-// 3: 4.
+// blocks, 467 at 4, 484 at 5; the order-4 MTTKRP 348, 350, 470).  FP64 orders 3
+// and 4: 4 (order 4 at rank 16 takes 66 registers uncapped, three blocks: 579
+// us a mode, 542 at four).
 template <typename FT, int NM, int LPN, int CH, bool PHI>
 constexpr int planned_min_blocks()
 {
     if (CH != 1) return 0;
-    if (sizeof(FT) != 4) return NM == 3 && !PHI ? 4 : 0;
+    if (sizeof(FT) != 4) return NM <= 4 ? 4 : 0;
     return NM == 3 && !PHI && LPN <= 16 ? 5 : 4;
 }
 
