@@ -313,11 +313,15 @@ static AprPhi apr_phi_kind(const altob_tensor* t, int R, size_t fsz, int max_inn
     if (v && !strcmp(v, "pre")) return PHI_PRE;
     if (v && !strcmp(v, "rows")) return PHI_ROWS;
     if (max_inner < 2) return PHI_OTF;
+    const double nnz = (double)t->nnz, rows = nnz * ((double)R * fsz + t->nmode * (8.0 + fsz) + 24.0);
+    // what an earlier solve left in the pool needs no question about free
+    // memory (cudaMemGetInfo can take milliseconds)
+    const size_t kept = pool_unused();
+    if (rows <= (double)kept) return PHI_ROWS;
     size_t fr = 0, tot = 0;
     if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) return PHI_OTF;
-    fr += pool_unused();
-    const double nnz = (double)t->nnz;
-    if (nnz * ((double)R * fsz + t->nmode * (8.0 + fsz) + 24.0) <= 0.25 * (double)fr) return PHI_ROWS;
+    fr += kept;
+    if (rows <= 0.25 * (double)fr) return PHI_ROWS;
     return nnz * R * fsz <= 0.25 * (double)fr ? PHI_PRE : PHI_OTF;
 }
 

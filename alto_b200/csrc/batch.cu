@@ -4,9 +4,10 @@
 // Every tensor of the batch keeps its own device model and follows exactly
 // the per-tensor algorithm of cpd_alto (include/cpd.hpp:43-186, as in
 // cpd.cu), but each step runs for all tensors in one launch:
-//   zero U_j | MTTKRP (one launch per shape class) | prepare |
+//   zero U_j | MTTKRP (one launch per shape class) |
 //   R x R solve (one CTA per tensor) | fused row update + column norms +
-//   Gram (+ fit inner product) | lambda, Gram scaling | U_j /= lambda
+//   Gram (+ fit inner product) | lambda, Gram scaling, U_j /= lambda (rank
+//   classes side by side)
 //   -- for every mode j; rank classes above 64 keep the separate passes
 //   (copy of the last mode, row apply + column norms, lambda, Gram of the
 //   normalised factor) --
@@ -92,13 +93,10 @@ __global__ void k_b_copym(const BDesc<FT>* __restrict__ d, BlkMap map, const int
     for (u64 e = (u64)bx * blockDim.x + threadIdx.x; e < n; e += (u64)nbx * blockDim.x) t.M[e] = t.U[j][e];
 }
 
+// Accumulators of mode j's update: column statistics, the Gram, the inner product.
 template <typename FT>
-__global__ void k_b_prep(const BDesc<FT>* __restrict__ d, const int* __restrict__ list,
-                         const int* __restrict__ active, int j, int nk)
+__device__ __forceinline__ void prep_body(const BDesc<FT>& t, int j, int nk)
 {
-    const int b = list[blockIdx.x];
-    if (!active[b]) return;
-    const BDesc<FT>& t = d[b];
     const int R = t.R;
     for (int r = threadIdx.x; r < R; r += blockDim.x) {
         t.colacc[r] = nk == NORM_MAX ? 1.0 : 0.0;
@@ -109,13 +107,24 @@ __global__ void k_b_prep(const BDesc<FT>* __restrict__ d, const int* __restrict_
 }
 
 template <typename FT>
+__global__ void k_b_prep(const BDesc<FT>* __restrict__ d, const int* __restrict__ list,
+                         const int* __restrict__ active, int j, int nk)
+{
+    const int b = list[blockIdx.x];
+    if (active[b]) prep_body(d[b], j, nk);
+}
+
+// The R x R solve, and the accumulators of the update that follows (the solve
+// reads the Grams of the other modes only).
+template <typename FT>
 __global__ void __launch_bounds__(DN_THREADS) k_b_solve(const BDesc<FT>* __restrict__ d,
                                                         const int* __restrict__ list,
-                                                        const int* __restrict__ active, int j)
+                                                        const int* __restrict__ active, int j, int nk)
 {
     const int b = list[blockIdx.x];
     if (!active[b]) return;
     const BDesc<FT>& t = d[b];
+    prep_body(t, j, nk);
     solve_body(t.G, t.nmode, j, t.R, t.W, t.info);
 }
 
@@ -146,34 +155,35 @@ __global__ void __launch_bounds__(AG_THREADS) k_b_apply_gram(const BDesc<FT>* __
                             j == t.nmode - 1 ? t.inner : nullptr, vec_ok, bx, nbx);
 }
 
-// U_j /= lambda after the fused pass
+// The end of the fused update (R <= 64): every block divides its rows of U_j
+// by the lambda it takes from the column statistics; a tensor's first block
+// also writes lambda, G_j /= lambda lambda^T and the inner product /= lambda.
 template <typename FT>
-__global__ void __launch_bounds__(DN_THREADS) k_b_div_cols(const BDesc<FT>* __restrict__ d, BlkMap map,
-                                                           const int* __restrict__ active, int j)
+__global__ void __launch_bounds__(DN_THREADS) k_b_finish(const BDesc<FT>* __restrict__ d, BlkMap map,
+                                                         const int* __restrict__ active, int j, int nk)
 {
     int bx, nbx;
     const int b = blk_owner(map, &bx, &nbx);
     if (!active[b]) return;
     const BDesc<FT>& t = d[b];
+    if (bx == 0)
+        lambda_finish_body(t.colacc, t.R, nk, t.lam, t.G + (size_t)j * t.R * t.R, j == t.nmode - 1 ? t.inner : nullptr);
     constexpr int V = 16 / sizeof(FT);
-    if (t.R % V == 0 && ((uintptr_t)t.U[j] & 15) == 0) div_cols_body<FT, V>(t.U[j], t.dims[j], t.R, t.lam, bx, nbx);
-    else div_cols_body<FT, 1>(t.U[j], t.dims[j], t.R, t.lam, bx, nbx);
+    const bool root = nk == NORM_2;
+    if (t.R % V == 0 && ((uintptr_t)t.U[j] & 15) == 0)
+        div_cols_body<FT, V>(t.U[j], t.dims[j], t.R, t.colacc, bx, nbx, root);
+    else div_cols_body<FT, 1>(t.U[j], t.dims[j], t.R, t.colacc, bx, nbx, root);
 }
 
-// lambda from the column statistics; after the fused pass (R <= 64) also
-// G_j /= lambda lambda^T and the inner product /= lambda
+// lambda from the column statistics of the tensors above rank 64
 template <typename FT>
 __global__ void k_b_lambda(const BDesc<FT>* __restrict__ d, const int* __restrict__ list,
-                           const int* __restrict__ active, int nk, int j)
+                           const int* __restrict__ active, int nk)
 {
     const int b = list[blockIdx.x];
     if (!active[b]) return;
     const BDesc<FT>& t = d[b];
-    if (t.R <= APPLY_GRAM_MAX_RANK) {
-        lambda_finish_body(t.colacc, t.R, nk, t.lam, t.G + (size_t)j * t.R * t.R,
-                           j == t.nmode - 1 ? t.inner : nullptr);
-        return;
-    }
+    if (t.R <= APPLY_GRAM_MAX_RANK) return;
     for (int r = threadIdx.x; r < t.R; r += blockDim.x) t.lam[r] = nk == NORM_2 ? sqrt(t.colacc[r]) : t.colacc[r];
 }
 
@@ -696,29 +706,61 @@ struct BatchImpl : BatchBase {
     static size_t smem_apply(int R) { return (size_t)(R * R + R) * sizeof(double); }
     static size_t smem_gram(int R) { return (size_t)(GR_ELEMS + 2 * R) * sizeof(double); }
 
-    // fused row update + Gram of mode j for the rank classes up to 64
-    void launch_apply_gram(int j, int nk, cudaStream_t st)
+    // fused row update + Gram and its end of mode j for rank class c (up to 64)
+    void launch_fused(int c, int j, int nk, cudaStream_t st)
     {
-        for (int c = 0; c < NRANK_CLASSES; ++c) {
-            if (!ncl[j][c] || !fused_class(c)) continue;
-            const BlkMap m = {d_clist[j][c], d_rowpre[j][c], ncl[j][c]};
-            const int g = nrowblk[j][c];
-            switch (c) {
-            case 0: k_b_apply_gram<FT, 1><<<g, AG_THREADS, apply_gram_smem<1>(), st>>>(d_desc, m, d_active, j, nk); break;
-            case 1: k_b_apply_gram<FT, 2><<<g, AG_THREADS, apply_gram_smem<2>(), st>>>(d_desc, m, d_active, j, nk); break;
-            case 2: k_b_apply_gram<FT, 4><<<g, AG_THREADS, apply_gram_smem<4>(), st>>>(d_desc, m, d_active, j, nk); break;
-            default: k_b_apply_gram<FT, 8><<<g, AG_THREADS, apply_gram_smem<8>(), st>>>(d_desc, m, d_active, j, nk); break;
-            }
+        const BlkMap m = {d_clist[j][c], d_rowpre[j][c], ncl[j][c]};
+        const int g = nrowblk[j][c];
+        switch (c) {
+        case 0: k_b_apply_gram<FT, 1><<<g, AG_THREADS, apply_gram_smem<1>(), st>>>(d_desc, m, d_active, j, nk); break;
+        case 1: k_b_apply_gram<FT, 2><<<g, AG_THREADS, apply_gram_smem<2>(), st>>>(d_desc, m, d_active, j, nk); break;
+        case 2: k_b_apply_gram<FT, 4><<<g, AG_THREADS, apply_gram_smem<4>(), st>>>(d_desc, m, d_active, j, nk); break;
+        default: k_b_apply_gram<FT, 8><<<g, AG_THREADS, apply_gram_smem<8>(), st>>>(d_desc, m, d_active, j, nk); break;
         }
+        k_b_finish<FT><<<g, DN_THREADS, cmaxR[c] * sizeof(double), st>>>(d_desc, m, d_active, j, nk);
     }
-    // U_j /= lambda for the fused rank classes (after k_b_lambda)
-    void launch_div_cols(int j, cudaStream_t st)
+    // branches of the dense update of mode j: the fused rank classes, and one
+    // for the classes above 64
+    altob_status dense_update(int j, int nk, const BlkMap& els, cudaStream_t st)
     {
+        const int* L = d_list[j];
+        const int n = nlist[j];
+        bool wide = false;
+        int classes = 0;
+        for (int c = 0; c < NRANK_CLASSES; ++c) {
+            wide = wide || (ncl[j][c] && !fused_class(c));
+            classes += ncl[j][c] && fused_class(c);
+        }
+        if (wide) k_b_copym<FT><<<nelblk[j], 256, 0, st>>>(d_desc, els, d_active, j);
+        k_b_solve<FT><<<n, DN_THREADS, smem_solve(), st>>>(d_desc, L, d_active, j, nk);
+        // the rank classes are independent and none fills the device: side by
+        // side on the forked streams, the first (or the wide ones) on st
+        const bool fork = classes + wide > 1;
+        if (fork) ALTOB_CUDA(cudaEventRecord(fork_ev, st));
+        int used = 0;
+        bool on_st = wide;
         for (int c = 0; c < NRANK_CLASSES; ++c) {
             if (!ncl[j][c] || !fused_class(c)) continue;
-            const BlkMap m = {d_clist[j][c], d_rowpre[j][c], ncl[j][c]};
-            k_b_div_cols<FT><<<nrowblk[j][c], DN_THREADS, cmaxR[c] * sizeof(double), st>>>(d_desc, m, d_active, j);
+            cudaStream_t fs = st;
+            if (on_st) {
+                fs = fork_st[used];
+                ALTOB_CUDA(cudaStreamWaitEvent(fs, fork_ev, 0));
+            }
+            launch_fused(c, j, nk, fs);
+            if (on_st) {
+                ALTOB_CUDA(cudaEventRecord(join_ev[used], fs));
+                ++used;
+            }
+            on_st = true;
         }
+        if (wide) {
+            launch_apply(j, nk, st);
+            k_b_lambda<FT><<<n, 128, 0, st>>>(d_desc, L, d_active, nk);
+            launch_gram(j, 1, st);
+        }
+        for (int i = 0; i < used; ++i) ALTOB_CUDA(cudaStreamWaitEvent(st, join_ev[i], 0));
+        ALTOB_LAUNCH_CHECK();
+        return ALTOB_OK;
     }
     static bool fused_class(int c) { return c <= 3; }  // rank classes up to R = 64
     // row kernels of mode j for the rank classes above 64, one launch per class
@@ -774,8 +816,7 @@ struct BatchImpl : BatchBase {
         for (int j = 0; j < maxN; ++j) {
             const int n = nlist[j];
             if (!n) continue;
-            const int* L = d_list[j];
-            const BlkMap els = {L, d_elpre[j], n};
+            const BlkMap els = {d_list[j], d_elpre[j], n};
             k_b_zero<FT><<<nelblk[j], 256, 0, st>>>(d_desc, els, d_active, j);
             // the launch groups of mode j are independent: spread them over
             // forked streams so one group's last wave overlaps the others
@@ -796,16 +837,8 @@ struct BatchImpl : BatchBase {
                 ALTOB_CUDA(cudaEventRecord(join_ev[i], fork_st[i]));
                 ALTOB_CUDA(cudaStreamWaitEvent(st, join_ev[i], 0));
             }
-            launches += 5 + 2 * row_launches(j);
-            k_b_copym<FT><<<nelblk[j], 256, 0, st>>>(d_desc, els, d_active, j);
-            k_b_prep<FT><<<n, 128, 0, st>>>(d_desc, L, d_active, j, nk);
-            k_b_solve<FT><<<n, DN_THREADS, smem_solve(), st>>>(d_desc, L, d_active, j);
-            launch_apply_gram(j, nk, st);
-            launch_apply(j, nk, st);
-            k_b_lambda<FT><<<n, 128, 0, st>>>(d_desc, L, d_active, nk, j);
-            launch_div_cols(j, st);
-            launch_gram(j, 1, st);
-            ALTOB_LAUNCH_CHECK();
+            launches += 2 + 2 * row_launches(j);
+            ALTOB_TRY(dense_update(j, nk, els, st));
         }
         k_b_fit<FT><<<count, DN_THREADS, 0, st>>>(d_desc, d_active, d_iters, eps, max_iters);
         ALTOB_LAUNCH_CHECK();

@@ -411,10 +411,15 @@ static altob_status run_tiled_vt(altob_tensor* t, int mode, void* const* dU, voi
         // a plan built by this call is not complete before the launch
         c.dependent = after_clear && (perm || had_plan);
         const u64 per_cta = a.ntiles / c.grid.x;
-        // one item per CTA: a hot-row table would pass every run on unchanged;
-        // in FP64, where it only saves contended atomics, it repays clearing
-        // and adding it up from about four tiles per CTA on
-        if (items <= cap || (sizeof(FT) == 8 && per_cta < 4)) a.hot = 0;
+        // FP32 keeps the table for a single tile too: it joins the pieces that
+        // the lane groups' stretches cut a long run into, which would each be
+        // an addition to the row (1M draws of a Zipf tensor through oidx:
+        // 2e-6 from FP64 without, 2.5e-7 with).  FP64 needs it for the contended
+        // atomics only, and it repays clearing and adding it up from about four
+        // tiles per CTA on.
+        if (sizeof(FT) == 8 && per_cta < 4) a.hot = 0;
+        // through oidx a long run is a row's whole range: the grouped kernel's line
+        if (perm && sizeof(FT) == 4) a.hot_minrun = GT_HOT_MINRUN;
         // an output of at most WHOLE_BYTES is kept whole by every CTA that
         // takes enough tiles to repay clearing the copy and adding it up
         if (!perm && t->dims[mode] * R * sizeof(FT) <= WHOLE_BYTES && t->dims[mode] <= 128 * per_cta && per_cta >= 2 &&
