@@ -334,9 +334,16 @@ struct PollFlag {
     cudaEvent_t ev[2] = {nullptr, nullptr};
     altob_status init()
     {
-        static thread_local int* word = nullptr;  // kept: eight bytes per host thread that ever solved
-        if (!word) ALTOB_CUDA(cudaHostAlloc((void**)&word, 2 * sizeof(int), cudaHostAllocPortable));
-        h = word;
+        struct Words {  // kept while the host thread lives
+            int* p = nullptr;
+            ~Words()
+            {
+                if (p) cudaFreeHost(p);
+            }
+        };
+        static thread_local Words words;
+        if (!words.p) ALTOB_CUDA(cudaHostAlloc((void**)&words.p, 2 * sizeof(int), cudaHostAllocPortable));
+        h = words.p;
         for (int k = 0; k < 2; ++k) ALTOB_CUDA(cudaEventCreateWithFlags(&ev[k], cudaEventDisableTiming));
         return ALTOB_OK;
     }

@@ -78,9 +78,9 @@ altob_status plan_tiled(const altob_tensor* t, u64 R, size_t fsz, bool aligned, 
     return ALTOB_OK;
 }
 
-// Per-CTA hot-row accumulator regions for a launch of `grid` CTAs (none when
-// the kernel has no hot-row slots; during stream capture a handle without a
-// large enough region runs without slots).
+// Per-CTA hot-row accumulator regions for a launch of `grid` CTAs.  When they
+// cannot be had (no memory, or a handle without a large enough region during
+// stream capture) the kernel runs without slots.
 template <typename FT>
 static altob_status set_hot_acc(altob_tensor* t, TiledArgs<FT>& a, unsigned grid, cudaStream_t st)
 {
@@ -88,13 +88,9 @@ static altob_status set_hot_acc(altob_tensor* t, TiledArgs<FT>& a, unsigned grid
     const int slots = a.whole ? a.whole : a.hot;
     if (!slots) return ALTOB_OK;
     void* p = nullptr;
-    const altob_status s = tensor_hotbuf(t, (size_t)grid * slots * a.R * sizeof(FT), &p, st);
-    if (s != ALTOB_OK && stream_capturing(st)) {
-        a.hot = a.whole = 0;
-        return ALTOB_OK;
-    }
+    if (tensor_hotbuf(t, (size_t)grid * slots * a.R * sizeof(FT), &p, st) != ALTOB_OK) a.hot = a.whole = 0;
     a.hot_acc = (FT*)p;
-    return s;
+    return ALTOB_OK;
 }
 
 // Tile plan of `mode` (k_tile_plan), built on the first call that needs it.

@@ -656,8 +656,9 @@ struct BatchTiles {
 };
 
 // Tensor of a global tile.  The tile prefixes and active flags of up to
-// BT_CACHE tensors are kept in shared memory: searched in global memory, the
-// seven dependent loads of every tile cost about 2 us of its 12.
+// BT_CACHE tensors are kept in shared memory: in global memory every tile
+// waited for about seven dependent loads (32 tensors, 4 iterations, together
+// with the rank classes side by side: 11.5 -> 10.3 ms).
 constexpr int BT_CACHE = 512;
 struct BatchLookup {
     u32 pre[BT_CACHE];
