@@ -270,13 +270,13 @@ static unsigned pad_grid(u64 rows, int R)
 
 template <typename FT, typename VT>
 static altob_status run_tiled_vt(altob_tensor* t, int mode, void* const* dU, void* dout, u64 R, bool phi,
-                                 double eps, const u32* perm, bool cache, bool after_clear, cudaStream_t st);
+                                 double eps, const u32* perm, bool cache, int flags, cudaStream_t st);
 
 // MTTKRP / Phi on padded copies of the factors; *ran = false when the copies
 // cannot be allocated (the caller then runs the scalar-row kernel).
 template <typename FT, typename VT>
 static altob_status run_padded(altob_tensor* t, int mode, void* const* dU, void* dout, u64 R, bool phi, double eps,
-                               const u32* perm, cudaStream_t st, bool* ran)
+                               const u32* perm, int flags, cudaStream_t st, bool* ran)
 {
     constexpr u64 V = 16 / sizeof(FT);
     const u64 Rp = (R + V - 1) / V * V;
@@ -309,18 +309,19 @@ static altob_status run_padded(altob_tensor* t, int mode, void* const* dU, void*
     pa.Rp = (int)Rp;
     k_pad_rows<FT><<<dim3(pad_grid(most, (int)Rp), n), 256, 0, st>>>(pa);
     ALTOB_LAUNCH_CHECK();
-    ALTOB_TRY((run_tiled_vt<FT, VT>(t, mode, pU, po, Rp, phi, eps, perm, true, false, st)));
+    ALTOB_TRY((run_tiled_vt<FT, VT>(t, mode, pU, po, Rp, phi, eps, perm, true, flags & MT_RUN_SUMS, st)));
     k_unpad_add<FT><<<pad_grid(t->dims[mode], (int)R), 256, 0, st>>>((FT*)dout, po, t->dims[mode], (int)R, (int)Rp);
     ALTOB_LAUNCH_CHECK();
     *ran = true;
     return ALTOB_OK;
 }
 
-// after_clear: the last launch on the stream is one that this call may overlap
-// (k_clear, or a solver's finish_cols): it writes nothing but factors.
+// flags: as mttkrp_device's; with MT_AFTER_CLEAR the last launch on the stream
+// is one that this call may overlap (k_clear, or a solver's finish_cols): it
+// writes nothing but factors.
 template <typename FT, typename VT>
 static altob_status run_tiled_vt(altob_tensor* t, int mode, void* const* dU, void* dout, u64 R, bool phi,
-                                 double eps, const u32* perm, bool cache, bool after_clear, cudaStream_t st)
+                                 double eps, const u32* perm, bool cache, int flags, cudaStream_t st)
 {
     const bool had_plan = t->d_plan[mode] != nullptr;
     bool aligned = ptr_aligned16(dout);
@@ -342,7 +343,7 @@ static altob_status run_tiled_vt(altob_tensor* t, int mode, void* const* dU, voi
         const u64 elems = rows * (R + 3);
         if (elems <= (4u << 20) ? 4 * t->nnz >= rows : elems <= (48u << 20) ? t->nnz >= rows : t->nnz >= 2 * rows) {
             bool ran = false;
-            ALTOB_TRY((run_padded<FT, VT>(t, mode, dU, dout, R, phi, eps, perm, st, &ran)));
+            ALTOB_TRY((run_padded<FT, VT>(t, mode, dU, dout, R, phi, eps, perm, flags, st, &ran)));
             if (ran) return ALTOB_OK;
         }
     }
@@ -405,7 +406,7 @@ static altob_status run_tiled_vt(altob_tensor* t, int mode, void* const* dU, voi
         const u64 items = a.ntiles << a.split_shift;
         c.grid = dim3((unsigned)std::max<u64>(1, std::min<u64>(items, cap)));
         // a plan built by this call is not complete before the launch
-        c.dependent = after_clear && (perm || had_plan);
+        c.dependent = (flags & MT_AFTER_CLEAR) && (perm || had_plan);
         const u64 per_cta = a.ntiles / c.grid.x;
         // FP32 keeps the table for a single tile too: it joins the pieces that
         // the lane groups' stretches cut a long run into, which would each be
@@ -418,7 +419,7 @@ static altob_status run_tiled_vt(altob_tensor* t, int mode, void* const* dU, voi
         if (perm && sizeof(FT) == 4) a.hot_minrun = GT_HOT_MINRUN;
         // an output of at most WHOLE_BYTES is kept whole by every CTA that
         // takes enough tiles to repay clearing the copy and adding it up
-        if (!perm && t->dims[mode] * R * sizeof(FT) <= WHOLE_BYTES && t->dims[mode] <= 128 * per_cta && per_cta >= 2 &&
+        if (!perm && !(flags & MT_RUN_SUMS) && t->dims[mode] * R * sizeof(FT) <= WHOLE_BYTES && t->dims[mode] <= 128 * per_cta && per_cta >= 2 &&
             env_int("ALTOB_HOT_ROWS", 1)) {
             a.hot = 0;
             a.whole = (int)t->dims[mode];
@@ -436,11 +437,11 @@ static altob_status run_tiled_vt(altob_tensor* t, int mode, void* const* dU, voi
 
 template <typename FT>
 static altob_status run_tiled(altob_tensor* t, int mode, void* const* dU, void* dout, u64 R, bool phi, double eps,
-                              const u32* perm, bool cache, bool after_clear, cudaStream_t st)
+                              const u32* perm, bool cache, int flags, cudaStream_t st)
 {
     const bool f64 = sizeof(FT) == 8;
-    if (t->vdt == ALTOB_U32) return run_tiled_vt<FT, u32>(t, mode, dU, dout, R, phi, eps, perm, cache, after_clear, st);
-    if ((t->vdt == ALTOB_F64) == f64) return run_tiled_vt<FT, FT>(t, mode, dU, dout, R, phi, eps, perm, cache, after_clear, st);
+    if (t->vdt == ALTOB_U32) return run_tiled_vt<FT, u32>(t, mode, dU, dout, R, phi, eps, perm, cache, flags, st);
+    if ((t->vdt == ALTOB_F64) == f64) return run_tiled_vt<FT, FT>(t, mode, dU, dout, R, phi, eps, perm, cache, flags, st);
     return fail(ALTOB_ERR_UNSUPPORTED, "stored value dtype does not match the compute dtype");
 }
 
@@ -516,7 +517,7 @@ static altob_status clear_output(const altob_tensor* t, void* p, u64 bytes, u64 
 }
 
 altob_status mttkrp_device(altob_tensor* t, int mode, altob_dtype ft, void* const* dU, u64 R, int accumulate,
-                           altob_algo algo, cudaStream_t st, bool after_clear)
+                           altob_algo algo, cudaStream_t st, int flags)
 {
     if (!t || !dU) return fail(ALTOB_ERR_ARG, "NULL argument");
     if (mode < 0 || mode >= t->nmode) return fail(ALTOB_ERR_ARG, "mode out of range");
@@ -527,8 +528,9 @@ altob_status mttkrp_device(altob_tensor* t, int mode, altob_dtype ft, void* cons
     const size_t fsz = ft == ALTOB_F64 ? 8 : 4;
     ALTOB_TRY(tensor_enter(t, st));
     TensorUse use(t, st);
-    after_clear = after_clear && !stream_capturing(st);
-    if (!accumulate) ALTOB_TRY(clear_output(t, dU[mode], t->dims[mode] * R * fsz, R, fsz, &after_clear, st));
+    bool overlap = (flags & MT_AFTER_CLEAR) && !stream_capturing(st);
+    if (!accumulate) ALTOB_TRY(clear_output(t, dU[mode], t->dims[mode] * R * fsz, R, fsz, &overlap, st));
+    flags = (flags & ~MT_AFTER_CLEAR) | (overlap ? MT_AFTER_CLEAR : 0);
     if (t->nnz == 0) return ALTOB_OK;
     algo = resolve_algo(t, mode, algo);
     const u32* perm = nullptr;
@@ -544,8 +546,8 @@ altob_status mttkrp_device(altob_tensor* t, int mode, altob_dtype ft, void* cons
         return ft == ALTOB_F64 ? run_atomic_cr<double>(t, mode, dU, R, st) : run_atomic_cr<float>(t, mode, dU, R, st);
     default: return fail(ALTOB_ERR_ARG, "unknown algorithm");
     }
-    return ft == ALTOB_F64 ? run_tiled<double>(t, mode, dU, dU[mode], R, false, 0.0, perm, cache, after_clear, st)
-                           : run_tiled<float>(t, mode, dU, dU[mode], R, false, 0.0, perm, cache, after_clear, st);
+    return ft == ALTOB_F64 ? run_tiled<double>(t, mode, dU, dU[mode], R, false, 0.0, perm, cache, flags, st)
+                           : run_tiled<float>(t, mode, dU, dU[mode], R, false, 0.0, perm, cache, flags, st);
 }
 
 altob_status phi_device(altob_tensor* t, int mode, altob_dtype ft, void* const* dU, u64 R, double eps,
@@ -560,8 +562,8 @@ altob_status phi_device(altob_tensor* t, int mode, altob_dtype ft, void* const* 
     bool dep = false;
     ALTOB_TRY(clear_output(t, dphi, t->dims[mode] * R * fsz, R, fsz, &dep, st));
     if (t->nnz == 0) return ALTOB_OK;
-    return ft == ALTOB_F64 ? run_tiled<double>(t, mode, dU, dphi, R, true, eps, nullptr, true, dep, st)
-                           : run_tiled<float>(t, mode, dU, dphi, R, true, eps, nullptr, true, dep, st);
+    return ft == ALTOB_F64 ? run_tiled<double>(t, mode, dU, dphi, R, true, eps, nullptr, true, dep ? MT_AFTER_CLEAR : 0, st)
+                           : run_tiled<float>(t, mode, dU, dphi, R, true, eps, nullptr, true, dep ? MT_AFTER_CLEAR : 0, st);
 }
 
 // ------------------------------------------------- precomputed Phi rows

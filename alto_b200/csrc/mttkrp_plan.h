@@ -17,10 +17,13 @@ altob_algo resolve_algo(const altob_tensor* t, int mode, altob_algo algo);
 // The tile plan of `mode` (built on first use; nullptr when plans are off or
 // cannot be allocated).
 const uint16_t* tensor_plan(altob_tensor* t, int mode, cudaStream_t st);
-// after_clear: the last launch on st is finish_cols, which the MTTKRP may
-// overlap up to its first read of a factor.
+// flags: MT_AFTER_CLEAR: the last launch on st is finish_cols, which the MTTKRP
+// may overlap up to its first read of a factor; MT_RUN_SUMS: every run is
+// added to the output itself, also where the output is short (no per-CTA
+// copies).
+enum { MT_AFTER_CLEAR = 1, MT_RUN_SUMS = 2 };
 altob_status mttkrp_device(altob_tensor* t, int mode, altob_dtype ft, void* const* dU, u64 R, int accumulate,
-                           altob_algo algo, cudaStream_t st, bool after_clear = false);
+                           altob_algo algo, cudaStream_t st, int flags = 0);
 altob_status phi_device(altob_tensor* t, int mode, altob_dtype ft, void* const* dU, u64 R, double eps,
                         void* dphi, cudaStream_t st);
 // Khatri-Rao rows of every nonzero for `mode` (nnz x R, ALTO order) and Phi
