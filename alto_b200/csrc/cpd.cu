@@ -85,9 +85,11 @@ static altob_status cpd_als_impl(altob_tensor* t, FT** U, FT* lam_out, int R, in
     for (int i = 0; i < max_iters; ++i) {
         const NormKind nk = i == 0 ? NORM_2 : NORM_MAX;
         for (int j = 0; j < N; ++j) {
-            // (after the first mode of a fused iteration the output is clear already)
+            // (after the first mode of a fused iteration the output is clear already;
+            // an FP32 model sums run by run, as the batched solver does, so that the
+            // fits of both stay alike)
             ALTOB_TRY(mttkrp_device(t, j, ft, (void* const*)U, (u64)R, fused && j > 0, ALTOB_ALGO_AUTO, st,
-                                    fused && j > 0 ? MT_AFTER_CLEAR : 0));
+                                    (fused && j > 0 ? MT_AFTER_CLEAR : 0) | (sizeof(FT) == 4 ? MT_RUN_SUMS : 0)));
             // a shard's partial MTTKRP summed over the GPUs; the dense update
             // below then runs on identical data on every GPU
             ALTOB_TRY(red(U[j], t->dims[j] * (u64)R, ft, ALTOB_REDUCE_SUM, st));
