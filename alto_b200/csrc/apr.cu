@@ -59,18 +59,34 @@ __global__ void k_mult(FT* __restrict__ B, const FT* __restrict__ Phi, u64 n)
         B[e] = (FT)((double)B[e] * (double)Phi[e]);
 }
 
-// The end of an inner round without the host: stops the mode's rounds when
-// the violation is below eps (every block reads the same value; one of them
-// sets the flag that later launches read), else B *= Phi, and Phi is zeroed
-// for the next round.
+// What a mode's queued inner rounds leave on the device: the violation of the
+// round in flight (two slots, so the next one is zero before its round
+// starts), that of the last round, how many rounds ran, and the flag that ends
+// them.  A fixed size: the limit on the rounds may be any int.
+struct Rounds {
+    double kkt[2];
+    double last;
+    int count, stop;
+};
+
+// The end of inner round r without the host: records it, and stops the mode's
+// rounds when the violation is below eps (every block reads the same value;
+// one of them sets the flag that later launches read), else B *= Phi, and Phi
+// is zeroed for the next round.
 template <typename FT, int VEC>
 __global__ void __launch_bounds__(256) k_round_end(FT* __restrict__ B, FT* __restrict__ Phi, u64 n,
-                                                   const double* __restrict__ kkt, double eps, int zero, int* stop)
+                                                   Rounds* rd, int r, double eps, int zero)
 {
     typedef typename VecT<FT, VEC>::T V;
-    if (*(volatile int*)stop) return;
-    if (*kkt < eps) {
-        if (blockIdx.x == 0 && threadIdx.x == 0) *(volatile int*)stop = 1;
+    if (*(volatile int*)&rd->stop) return;
+    const double kkt = rd->kkt[r & 1];
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        rd->kkt[(r + 1) & 1] = 0.0;
+        rd->last = kkt;
+        rd->count = r + 1;
+    }
+    if (kkt < eps) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) *(volatile int*)&rd->stop = 1;
         return;
     }
     for (u64 e = (u64)blockIdx.x * blockDim.x + threadIdx.x; e < n / VEC; e += (u64)gridDim.x * blockDim.x) {
@@ -100,15 +116,14 @@ static altob_status launch_kkt(FT* B, const FT* Phi, u64 n, double* kkt, int mul
 }
 
 template <typename FT>
-static altob_status launch_round_end(FT* B, FT* Phi, u64 n, const double* kkt, double eps, int zero, int* stop,
-                                     cudaStream_t st)
+static altob_status launch_round_end(FT* B, FT* Phi, u64 n, Rounds* rd, int r, double eps, int zero, cudaStream_t st)
 {
     constexpr int V = 16 / sizeof(FT);
     const bool vec = ptr_aligned16(B) && n % V == 0;
     const u64 pieces = vec ? n / V : n;
     const int g = (int)std::max<u64>(1, std::min<u64>((pieces + 511) / 512, (u64)num_sms() * 8));
-    if (vec) k_round_end<FT, V><<<g, 256, 0, st>>>(B, Phi, n, kkt, eps, zero, stop);
-    else k_round_end<FT, 1><<<g, 256, 0, st>>>(B, Phi, n, kkt, eps, zero, stop);
+    if (vec) k_round_end<FT, V><<<g, 256, 0, st>>>(B, Phi, n, rd, r, eps, zero);
+    else k_round_end<FT, 1><<<g, 256, 0, st>>>(B, Phi, n, rd, r, eps, zero);
     ALTOB_LAUNCH_CHECK();
     return ALTOB_OK;
 }
@@ -272,7 +287,8 @@ static altob_status loglik_sum(const altob_tensor* t, FT** U, int R, double eps,
 }
 
 struct AprScratch {
-    double *lam, *colacc, *llacc, *rounds, *kkt, *G, *inner, *fit, *normAT;
+    double *lam, *colacc, *llacc, *kkt, *G, *inner, *fit, *normAT;
+    Rounds* rounds;  // one per mode
     int* info;
 };
 
@@ -367,7 +383,8 @@ static altob_status cp_apr_impl(altob_tensor* t, FT** U, FT* lam_io, int R, int 
         phi_off[n] = phi_elems;
         phi_elems += (t->dims[n] * R + 63) & ~(size_t)63;
     }
-    size_t nd = 5 * (size_t)R + (size_t)N * R * R + (size_t)N * (max_inner + 1) + 16;
+    constexpr size_t RD = sizeof(Rounds) / sizeof(double);
+    size_t nd = 5 * (size_t)R + (size_t)N * R * R + (size_t)N * RD + 16;
     size_t bytes = nd * sizeof(double) + 256 + phi_elems * sizeof(FT) + 256;
     void* base = nullptr;
     ALTOB_TRY(tensor_scratch(t, bytes, &base));
@@ -387,8 +404,8 @@ static altob_status cp_apr_impl(altob_tensor* t, FT** U, FT* lam_io, int R, int 
     s.normAT = d++;
     s.llacc = d;
     d += R + 2;
-    s.rounds = d;
-    d += (size_t)N * (max_inner + 1);
+    s.rounds = (Rounds*)d;
+    d += (size_t)N * RD;
     s.info = (int*)d;
     d += 2;
     FT* phi_base = (FT*)(((uintptr_t)d + 255) & ~(uintptr_t)255);
@@ -466,7 +483,7 @@ static altob_status cp_apr_impl(altob_tensor* t, FT** U, FT* lam_io, int R, int 
     const bool queued = rows && !env_int("ALTOB_PHI_TMA", 0);
     PollFlag poll;
     if (queued) ALTOB_TRY(poll.init());
-    std::vector<double> hrounds((size_t)N * (max_inner + 1));
+    std::vector<Rounds> hrounds(N);
     int iter;
     for (iter = 0; iter < max_iters; ++iter) {
         bool converged = false;
@@ -488,17 +505,17 @@ static altob_status cp_apr_impl(altob_tensor* t, FT** U, FT* lam_io, int R, int 
                 // once.  The stop flag is polled one group of rounds behind,
                 // so the device never waits for the host and few empty rounds
                 // are queued.
-                double* kk = s.rounds + (size_t)n * (max_inner + 1);
-                int* stop = (int*)(kk + max_inner);
+                Rounds* rd = s.rounds + n;
+                int* stop = &rd->stop;
                 const double stop_eps = dobench ? -1.0 : eps;  // bench mode: all rounds
-                ALTOB_CUDA(cudaMemsetAsync(kk, 0, (size_t)(max_inner + 1) * sizeof(double), st));
+                ALTOB_CUDA(cudaMemsetAsync(rd, 0, sizeof(Rounds), st));
                 ALTOB_CUDA(cudaMemsetAsync(Phi[n], 0, sz * sizeof(FT), st));
                 int group = 0;
                 for (int r = 0; r < max_inner; ++r) {
                     ALTOB_TRY(phi_rows_device(t, n, ft, pi, rows + (size_t)n * nnzp, svals + (size_t)n * nnzp, B, (u64)R,
                                               eps_div_zero, Phi[n], st, true, stop));
-                    ALTOB_TRY(launch_kkt<FT>(B, Phi[n], sz, kk + r, 0, stop, st));
-                    ALTOB_TRY(launch_round_end<FT>(B, Phi[n], sz, kk + r, stop_eps, r + 1 < max_inner, stop, st));
+                    ALTOB_TRY(launch_kkt<FT>(B, Phi[n], sz, rd->kkt + (r & 1), 0, stop, st));
+                    ALTOB_TRY(launch_round_end<FT>(B, Phi[n], sz, rd, r, stop_eps, r + 1 < max_inner, st));
                     if (dobench || r + 1 == max_inner || (r + 1) % APR_GROUP) continue;
                     ALTOB_CUDA(cudaMemcpyAsync((int*)poll.h + group % 2, stop, sizeof(int), cudaMemcpyDeviceToHost, st));
                     ALTOB_CUDA(cudaEventRecord(poll.ev[group % 2], st));
@@ -538,16 +555,11 @@ static altob_status cp_apr_impl(altob_tensor* t, FT** U, FT* lam_io, int R, int 
             ALTOB_TRY(div_cols<FT>(B, t->dims[n], R, s.colacc, s.lam, true, st));
         }
         if (queued) {
-            // the violations of every round and mode tell which round was the last
-            ALTOB_CUDA(cudaMemcpyAsync(hrounds.data(), s.rounds, hrounds.size() * sizeof(double), cudaMemcpyDeviceToHost,
-                                       st));
+            ALTOB_CUDA(cudaMemcpyAsync(hrounds.data(), s.rounds, N * sizeof(Rounds), cudaMemcpyDeviceToHost, st));
             ALTOB_CUDA(cudaStreamSynchronize(st));
             for (int n = 0; n < N; ++n) {
-                const double* kk = hrounds.data() + (size_t)n * (max_inner + 1);
-                int r = 0;
-                while (r + 1 < max_inner && (dobench || !(kk[r] < eps))) ++r;
-                ninner[iter] += r + 1;
-                kmode[n] = kk[r];
+                ninner[iter] += hrounds[n].count;
+                kmode[n] = hrounds[n].last;
             }
         } else if (dobench) {
             ALTOB_CUDA(cudaMemcpyAsync(kmode.data(), s.kkt, N * sizeof(double), cudaMemcpyDeviceToHost, st));
