@@ -348,7 +348,7 @@ constexpr int APR_GROUP = 2;
 struct PollFlag {
     volatile int* h = nullptr;
     cudaEvent_t ev[2] = {nullptr, nullptr};
-    altob_status init()
+    bool init()
     {
         struct Words {  // kept while the host thread lives
             int* p = nullptr;
@@ -358,10 +358,13 @@ struct PollFlag {
             }
         };
         static thread_local Words words;
-        if (!words.p) ALTOB_CUDA(cudaHostAlloc((void**)&words.p, 2 * sizeof(int), cudaHostAllocPortable));
+        cudaError_t e = cudaSuccess;
+        if (!words.p) e = cudaHostAlloc((void**)&words.p, 2 * sizeof(int), cudaHostAllocPortable);
+        if (e != cudaSuccess) words.p = nullptr;
         h = words.p;
-        for (int k = 0; k < 2; ++k) ALTOB_CUDA(cudaEventCreateWithFlags(&ev[k], cudaEventDisableTiming));
-        return ALTOB_OK;
+        for (int k = 0; k < 2 && e == cudaSuccess; ++k) e = cudaEventCreateWithFlags(&ev[k], cudaEventDisableTiming);
+        if (e != cudaSuccess) cudaGetLastError();
+        return e == cudaSuccess;
     }
     ~PollFlag()
     {
@@ -479,10 +482,10 @@ static altob_status cp_apr_impl(altob_tensor* t, FT** U, FT* lam_io, int R, int 
         pi_free.p = pi;
     }
     // rounds without the host in between: the row-ordered stream through the
-    // register-staged kernel (the opt-in bulk-copy kernel takes no stop flag)
-    const bool queued = rows && !env_int("ALTOB_PHI_TMA", 0);
+    // register-staged kernel (the opt-in bulk-copy kernel takes no stop flag),
+    // while the host can have its poll words; else the host drives every round
     PollFlag poll;
-    if (queued) ALTOB_TRY(poll.init());
+    const bool queued = rows && !env_int("ALTOB_PHI_TMA", 0) && poll.init();
     std::vector<Rounds> hrounds(N);
     int iter;
     for (iter = 0; iter < max_iters; ++iter) {
