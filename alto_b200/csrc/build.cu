@@ -126,31 +126,33 @@ bool stream_capturing(cudaStream_t st)
 }
 
 // Buffers that outlive the call are never grown while st is being captured:
-// the allocation would belong to the graph.
-static altob_status grow_buf(void** buf, size_t* have, size_t bytes, void** out, cudaStream_t st)
+// the allocation would belong to the graph.  A buffer that a captured call
+// has used stays allocated until the handle is destroyed, since the graph
+// keeps its address: it is set aside when a later call needs a larger one.
+static altob_status grow_buf(altob_tensor* t, HandleBuf* b, size_t bytes, void** out, cudaStream_t st)
 {
-    if (bytes > *have) {
-        if (stream_capturing(st)) return fail(ALTOB_ERR_NOMEM, "a handle's buffer cannot grow during stream capture");
-        if (*buf) {
-            dfree(*buf);
-            *buf = nullptr;
-            *have = 0;
-        }
-        ALTOB_TRY(dmalloc(buf, bytes));
-        *have = bytes;
+    const bool cap = stream_capturing(st);
+    if (bytes > b->bytes) {
+        if (cap) return fail(ALTOB_ERR_NOMEM, "a handle's buffer cannot grow during stream capture");
+        if (b->in_graph) t->set_aside.push_back({b->p, b->bytes});
+        else dfree(b->p);
+        *b = HandleBuf();
+        ALTOB_TRY(dmalloc(&b->p, bytes));
+        b->bytes = bytes;
     }
-    *out = *buf;
+    b->in_graph = b->in_graph || cap;
+    *out = b->p;
     return ALTOB_OK;
 }
 
 altob_status tensor_hotbuf(altob_tensor* t, size_t bytes, void** out, cudaStream_t st)
 {
-    return grow_buf(&t->hotbuf, &t->hotbuf_bytes, bytes, out, st);
+    return grow_buf(t, &t->hotbuf, bytes, out, st);
 }
 
 altob_status tensor_padbuf(altob_tensor* t, size_t bytes, void** out, cudaStream_t st)
 {
-    return grow_buf(&t->padbuf, &t->padbuf_bytes, bytes, out, st);
+    return grow_buf(t, &t->padbuf, bytes, out, st);
 }
 
 altob_status tensor_enter(altob_tensor* t, cudaStream_t st)
@@ -1001,8 +1003,9 @@ altob_status altob_destroy(altob_tensor* t)
     for (int n = 0; n < ALTOB_MAX_MODES; ++n) dfree(t->d_oidx[n]);
     for (int n = 0; n < ALTOB_MAX_MODES; ++n) dfree(t->d_plan[n]);
     dfree(t->scratch);
-    dfree(t->hotbuf);
-    dfree(t->padbuf);
+    dfree(t->hotbuf.p);
+    dfree(t->padbuf.p);
+    for (const altob::HandleBuf& b : t->set_aside) dfree(b.p);
     dfree(t->d_tma_err);
     if (t->h_tma_err) {
         cudaStreamSynchronize(0);  // the flag's last copy was ordered before the frees above

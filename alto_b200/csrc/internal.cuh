@@ -178,6 +178,13 @@ __device__ __forceinline__ u64 key_hi(const KeySrc& k, u64 i)
 
 // ------------------------------------------------------------- tensor
 
+// A device buffer that a handle keeps between calls.
+struct HandleBuf {
+    void* p = nullptr;
+    size_t bytes = 0;
+    bool in_graph = false;  // a captured call has used it
+};
+
 }  // namespace altob
 
 struct altob_tensor {
@@ -208,12 +215,10 @@ struct altob_tensor {
     // cached scratch (grown on demand, freed with the handle)
     void* scratch = nullptr;
     size_t scratch_bytes = 0;
-    // per-CTA hot-row accumulators of the grouped kernel (grown on demand)
-    void* hotbuf = nullptr;
-    size_t hotbuf_bytes = 0;
-    // padded factor copies of ranks without vector rows (grown on demand)
-    void* padbuf = nullptr;
-    size_t padbuf_bytes = 0;
+    // per-CTA accumulators of the grouped and planned kernels, and padded
+    // factor copies of ranks without vector rows (grown on demand)
+    altob::HandleBuf hotbuf, padbuf;
+    std::vector<altob::HandleBuf> set_aside;  // outgrown, but a captured call's graph has their address
     // tile plans of the planned MTTKRP kernel, one per mode (built on first use)
     uint16_t* d_plan[ALTOB_MAX_MODES] = {nullptr};
     // the TMA-staged kernel's wait-limit flag: on the device, and a pinned

@@ -273,7 +273,9 @@ static altob_status run_tiled_vt(altob_tensor* t, int mode, void* const* dU, voi
                                  double eps, const u32* perm, bool cache, int flags, cudaStream_t st);
 
 // MTTKRP / Phi on padded copies of the factors; *ran = false when the copies
-// cannot be allocated (the caller then runs the scalar-row kernel).
+// cannot be allocated (the caller then runs the scalar-row kernel), and during
+// stream capture: the copies belong to the handle, and graphs of one handle
+// may be replayed side by side.
 template <typename FT, typename VT>
 static altob_status run_padded(altob_tensor* t, int mode, void* const* dU, void* dout, u64 R, bool phi, double eps,
                                const u32* perm, int flags, cudaStream_t st, bool* ran)
@@ -281,6 +283,7 @@ static altob_status run_padded(altob_tensor* t, int mode, void* const* dU, void*
     constexpr u64 V = 16 / sizeof(FT);
     const u64 Rp = (R + V - 1) / V * V;
     *ran = false;
+    if (stream_capturing(st)) return ALTOB_OK;
     u64 elems = 0, most = 0, off[ALTOB_MAX_MODES], out_off = 0;
     for (int m = 0; m < t->nmode; ++m) {
         off[m] = elems;
@@ -414,13 +417,16 @@ static altob_status run_tiled_vt(altob_tensor* t, int mode, void* const* dU, voi
         // 2e-6 from FP64 without, 2.5e-7 with).  FP64 needs it for the contended
         // atomics only, and it repays clearing and adding it up from about four
         // tiles per CTA on.
-        if (sizeof(FT) == 8 && per_cta < 4) a.hot = 0;
+        // FP64 captures run without accumulators: they belong to the handle,
+        // and graphs of one handle may be replayed side by side.
+        const bool apart = sizeof(FT) == 8 && stream_capturing(st);
+        if (apart || (sizeof(FT) == 8 && per_cta < 4)) a.hot = 0;
         // through oidx a long run is a row's whole range: the grouped kernel's line
         if (perm && sizeof(FT) == 4) a.hot_minrun = GT_HOT_MINRUN;
         // an output of at most WHOLE_BYTES is kept whole by every CTA that
         // takes enough tiles to repay clearing the copy and adding it up
-        if (!perm && !(flags & MT_RUN_SUMS) && t->dims[mode] * R * sizeof(FT) <= WHOLE_BYTES && t->dims[mode] <= 128 * per_cta && per_cta >= 2 &&
-            env_int("ALTOB_HOT_ROWS", 1)) {
+        if (!apart && !perm && !(flags & MT_RUN_SUMS) && t->dims[mode] * R * sizeof(FT) <= WHOLE_BYTES &&
+            t->dims[mode] <= 128 * per_cta && per_cta >= 2 && env_int("ALTOB_HOT_ROWS", 1)) {
             a.hot = 0;
             a.whole = (int)t->dims[mode];
         }
