@@ -401,11 +401,22 @@ static altob_status run_tiled_vt(altob_tensor* t, int mode, void* const* dU, voi
         if (bps < 1) return fail(ALTOB_ERR_UNSUPPORTED, "planned MTTKRP kernel does not fit on an SM");
         // a tensor with fewer tiles than resident CTAs shares each tile among
         // 2^split_shift CTAs (at least two records per lane group each):
-        // 40,000 nonzeros, order 3, rank 16, FP64: 8.0 -> 6.2 us a mode;
-        // 150,001 nonzeros, order 5, rank 64, FP32: 25 -> 15
+        // 150,001 nonzeros, order 5, rank 64, FP32: 25 -> 15 us a mode.
+        // A shorter stretch cuts the runs of a short mode into more pieces,
+        // all added to the same few rows: halving it to s records saves about
+        // 0.165 s us of a lane group's walk and costs about 25 us x tiles /
+        // (s x rows) in the row's additions, so it goes on while s^2 rows >=
+        // 160 tiles (100,000 nonzeros, FP64: 30 rows at rank 4 take 22.9 us
+        // unsplit and 63.9 in quarters, 100 rows 13.2 and 25.0, 40,000 rows
+        // of rank 16 14.6 and 12.5; 40,000 nonzeros, 100 rows, rank 16: 12.5
+        // unsplit, 9.8 in halves, 10.7 in eighths)
         const u64 cap = (u64)bps * num_sms();
         const int ipg = planned_ipg(PT_TILE, c.lpn);
-        while ((a.ntiles << (a.split_shift + 1)) <= cap && (ipg >> (a.split_shift + 1)) >= 2) ++a.split_shift;
+        auto may_split = [&](int shift) {
+            const u64 s = (u64)(ipg >> shift);
+            return (a.ntiles << shift) <= cap && s >= 2 && s * s * t->dims[mode] >= 160 * a.ntiles;
+        };
+        while (may_split(a.split_shift + 1)) ++a.split_shift;
         const u64 items = a.ntiles << a.split_shift;
         c.grid = dim3((unsigned)std::max<u64>(1, std::min<u64>(items, cap)));
         // a plan built by this call is not complete before the launch
