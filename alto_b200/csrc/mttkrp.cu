@@ -498,10 +498,11 @@ altob_algo resolve_algo(const altob_tensor* t, int mode, altob_algo algo)
     return ALTOB_ALGO_ATOMIC;
 }
 
-// Clears an output and lets the kernel after it start meanwhile.
-__global__ void __launch_bounds__(256) k_clear(u32* p, u64 n)
+// Clears an output and lets the kernel after it start: at once (early), or
+// when the stores are issued.
+__global__ void __launch_bounds__(256) k_clear(u32* p, u64 n, bool early)
 {
-    grid_trigger();
+    if (early) grid_trigger();
     const u64 t = (u64)blockIdx.x * blockDim.x + threadIdx.x, step = (u64)gridDim.x * blockDim.x;
     if (((uintptr_t)p & 15) == 0) {
         for (u64 e = t; e < n / 4; e += step) reinterpret_cast<uint4*>(p)[e] = make_uint4(0, 0, 0, 0);
@@ -509,15 +510,28 @@ __global__ void __launch_bounds__(256) k_clear(u32* p, u64 n)
     } else {
         for (u64 e = t; e < n; e += step) p[e] = 0;
     }
+    if (!early) grid_trigger();
 }
+
+// Largest output (bytes) whose clearing the kernel after it overlaps from the
+// start, unless there are at most two tiles per SM (the tiles are then shared
+// and scattered by several CTAs, a longer time before the first addition:
+// 150,001 nonzeros of order 5, rank 64, FP32, 10.5 MB 21.0 us from the start,
+// 23.0 after the stores; 250,000 of order 3, rank 64, FP64 50.3 and 59.5).  A CTA that starts on an SM beside a block of k_clear finds that
+// block's split of shared memory and L1, and the SM then holds fewer CTAs for
+// the whole launch.  Few blocks (4096 words each) leave most SMs free of
+// that: 1M nonzeros, 1000 x 800 x 600, rank 32, FP64 (256 KB) 40.9 us a mode
+// so, 43.5 started after the stores, 44.7 behind a memset.  Many do not: 1M
+// nonzeros, 20,000 x 15,000 x 10,000, rank 64, FP32 (5.1 MB) 76.2, 59.6 and
+// 61.8; 400,000 of order 5, rank 64, 640 KB 42.3, 37.5 and 40.3.
+constexpr u64 CLEAR_EARLY_BYTES = 512 * 1024;
 
 // Zeroes an output for the planned kernel that follows; *overlap tells whether
 // that kernel may start meanwhile.  Worth it where the kernel outlasts the
 // host's two launches (about 8 us, 32 MB of gathered rows; below, a memset and
 // an ordinary launch cost the host less: 40,000 nonzeros of order 3 at rank 16,
 // FP64, 28.3 against 31.9 us a sweep) and the output is small against the
-// gathers (1M nonzeros 88 -> 84 us a sweep, 150,001 of order 5 at rank 64 99 ->
-// 90; clearing 614 MB outputs so took 6943 against 6840).
+// gathers (clearing 614 MB outputs so took 6943 against 6840).
 static altob_status clear_output(const altob_tensor* t, void* p, u64 bytes, u64 R, size_t fsz, bool* overlap,
                                  cudaStream_t st)
 {
@@ -527,7 +541,9 @@ static altob_status clear_output(const altob_tensor* t, void* p, u64 bytes, u64 
         return ALTOB_OK;
     }
     const u64 n = bytes / 4;  // factors are whole 4-byte words
-    k_clear<<<(unsigned)std::max<u64>(1, std::min<u64>((n + 4095) / 4096, (u64)num_sms() * 8)), 256, 0, st>>>((u32*)p, n);
+    const unsigned grid = (unsigned)std::max<u64>(1, std::min<u64>((n + 4095) / 4096, (u64)num_sms() * 8));
+    const bool early = bytes <= CLEAR_EARLY_BYTES || t->nnz <= 2ull * PT_TILE * num_sms();
+    k_clear<<<grid, 256, 0, st>>>((u32*)p, n, early);
     ALTOB_LAUNCH_CHECK();
     *overlap = true;
     return ALTOB_OK;
