@@ -344,7 +344,18 @@ static altob_status run_tiled_vt(altob_tensor* t, int mode, void* const* dU, voi
         // nonzeros 186 -> 98; 1.5M rows and nonzeros, rank 25 925 -> 678, but
         // rank 50 1122 -> 1183; 3M nonzeros, rank 50 2022 -> 1708.
         const u64 elems = rows * (R + 3);
-        if (elems <= (4u << 20) ? 4 * t->nnz >= rows : elems <= (48u << 20) ? t->nnz >= rows : t->nnz >= 2 * rows) {
+        bool pad = elems <= (4u << 20) ? 4 * t->nnz >= rows : elems <= (48u << 20) ? t->nnz >= rows : t->nnz >= 2 * rows;
+        // The MTTKRP in FP64 above rank 64: the vector kernel's two chunks per
+        // row are no faster than the scalar rows once the gathered factors
+        // outgrow the L1 caches, except at order 5 (four gathers per nonzero).
+        // Scalar -> padded, us a mode: 1M nonzeros of order 3, 45,000 rows,
+        // rank 67 214 -> 229, rank 127 272 -> 395; 6M 1038 -> 927 and 1297 ->
+        // 1784; 2,400 rows, rank 127 182 -> 139; 2M nonzeros of order 5,
+        // 71,000 rows, rank 127 827 -> 735, but 150,001 72 -> 108.
+        if (sizeof(FT) == 8 && R > 64 && !phi &&
+            (R <= 72 ? elems > (4u << 20) : (rows - t->dims[mode]) * (R + 3) > (1u << 18)))
+            pad = t->nmode == 5 ? t->nnz >= 8 * rows : R <= 72 && t->nnz >= 64 * rows;
+        if (pad) {
             bool ran = false;
             ALTOB_TRY((run_padded<FT, VT>(t, mode, dU, dout, R, phi, eps, perm, flags, st, &ran)));
             if (ran) return ALTOB_OK;
