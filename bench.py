@@ -98,6 +98,20 @@ def parse():
     return p.parse_args()
 
 
+def finite_errors(got, want):
+    """|got - want| of the pairs that are finite on both sides, and how many
+    of each side are not: an FP32 solve of a nearly singular model can end in
+    NaN, which max() would drop or spread depending on where it stands."""
+    got, want = np.asarray(got, np.float64), np.asarray(want, np.float64)
+    ok = np.isfinite(got) & np.isfinite(want)
+    return np.abs(got[ok] - want[ok]), int(np.sum(~np.isfinite(got))), int(np.sum(~np.isfinite(want)))
+
+
+def stat(fn, x):
+    """fn of the errors, None when there are none."""
+    return float(fn(x)) if len(x) else None
+
+
 # ------------------------------------------------------------ data (torch)
 
 def zipf_tensor_torch(dims, draws, s, seed, device):
@@ -602,12 +616,12 @@ def run_batch(args):
         bms = b0.elapsed_time(b1)
         base = {"value": args.batch_count / (bms / 1e3), "unit": "solves/s", "ms": bms,
                 "path": "altob_cpd_als, FP64 model and values, one tensor after another on one stream"}
-        fd = [abs(fits32[k][iters - 1] - f64[k][-1]) for k in range(len(shapes))]
-        fit_err = {"final_within_tol": int(sum(d < 1e-4 for d in fd)), "of": len(fd),
-                   "final_median_abs": float(np.median(fd)),
-                   "final_max_abs": float(max(fd)),
-                   "all_iters_max_abs": float(max(np.max(np.abs(fits32[k][:iters] - f64[k])) for k in
-                                                  range(len(shapes)))),
+        fd, bad32, bad64 = finite_errors([fits32[k][iters - 1] for k in range(len(shapes))], [f[-1] for f in f64])
+        every = finite_errors(np.concatenate([fits32[k][:iters] for k in range(len(shapes))]), np.concatenate(f64))[0]
+        fit_err = {"final_within_tol": int(np.sum(fd < 1e-4)), "of": len(shapes),
+                   "nonfinite_f32": bad32, "nonfinite_f64": bad64,
+                   "final_median_abs": stat(np.median, fd), "final_max_abs": stat(np.max, fd),
+                   "all_iters_max_abs": stat(np.max, every),
                    "tolerance": 1e-4}
     b.close()
     line = {"metric": "batched_cpals_solves_per_s", "value": value, "unit": "solves/s", "n_gpus": ws,
@@ -688,14 +702,18 @@ def run_serve(args):
         for kind in ("als", "apr"):
             base[f"{kind}_service_s"] = float(sum(b["t_end"] - b["t_start"] for (k, *_), b in zip(inputs, bres)
                                                   if k == kind))
-        als_d = [abs(a["fit"] - b["fit"]) for (kind, *_), a, b in zip(inputs, res, bres) if kind == "als"]
-        apr_d = [abs(a["loglik"] - b["loglik"]) / max(1e-300, abs(b["loglik"]))
-                 for (kind, *_), a, b in zip(inputs, res, bres) if kind == "apr"]
-        agree = {"als_fit_within_1e-4": int(sum(d < 1e-4 for d in als_d)), "als": len(als_d),
-                 "als_fit_max_abs": float(max(als_d)) if als_d else None,
-                 "als_fit_median_abs": float(np.median(als_d)) if als_d else None,
-                 "apr_loglik_within_1e-4_rel": int(sum(d < 1e-4 for d in apr_d)), "apr": len(apr_d),
-                 "apr_loglik_max_rel": float(max(apr_d)) if apr_d else None}
+        def pairs(what, key):
+            return [[r[key] for (kind, *_), r in zip(inputs, rs) if kind == what] for rs in (res, bres)]
+
+        als_d, als_bad, als_bad64 = finite_errors(*pairs("als", "fit"))
+        apr, apr64 = pairs("apr", "loglik")
+        apr_d, apr_bad, apr_bad64 = finite_errors(np.array(apr) / np.maximum(1e-300, np.abs(apr64)),
+                                                  np.array(apr64) / np.maximum(1e-300, np.abs(apr64)))
+        agree = {"als_fit_within_1e-4": int(np.sum(als_d < 1e-4)), "als": sum(1 for x in inputs if x[0] == "als"),
+                 "als_fit_max_abs": stat(np.max, als_d), "als_fit_median_abs": stat(np.median, als_d),
+                 "apr_loglik_within_1e-4_rel": int(np.sum(apr_d < 1e-4)), "apr": len(apr),
+                 "apr_loglik_max_rel": stat(np.max, apr_d),
+                 "nonfinite_f32": als_bad + apr_bad, "nonfinite_f64": als_bad64 + apr_bad64}
     line = {"metric": "served_solves_per_s", "value": summ["solves_per_s"], "unit": "solves/s", "n_gpus": ws,
             "steps": 1, "warmup": 1, "ms_per_step": summ["makespan_s"] * 1e3, "higher_is_better": True,
             "scaling": "weak", "vs_baseline": None, "dtype": "f32 (FP64 Gram/solve/fit/KKT/LL)",
