@@ -59,14 +59,20 @@ static u64 footprint(const altob_request& r)
     u64 rows = 0;
     for (int m = 0; m < r.nmode; ++m) rows += r.dims[m];
     const u64 build_peak = r.nnz * 48;                       // keys, payloads, ping-pong buffers
-    const u64 resident = r.nnz * (8 + vsz + 4 * (u64)r.nmode);  // key, value, oidx
+    const u64 resident = r.nnz * (8 + vsz + 4 * (u64)r.nmode);  // key, value, oidx or tile plan
+    // what a handle keeps beside them: padded factor copies of a rank that is no
+    // vector multiple, and a copy of a short output (at most 64 KB) per CTA of
+    // two tiles or more
+    const u64 V = 16 / fsz;
+    const u64 kept = (r.rank % V ? rows * ((r.rank + V - 1) / V * V) * fsz : 0) +
+                     std::min<u64>(r.nnz / 2048 * (64ull << 10), 48ull << 20);
     const u64 model = rows * r.rank * fsz * (r.kind == ALTOB_REQ_CP_APR ? 4 : 2) +
                       r.dims[r.nmode - 1] * r.rank * fsz + (u64)r.nmode * r.rank * r.rank * 8 * 2;
     const bool apr = r.kind == ALTOB_REQ_CP_APR;
     const u64 pi = apr ? r.nnz * r.rank * fsz : 0;  // precomputed Khatri-Rao rows
     // row-ordered Phi stream (row, value, position per mode) and its sort scratch
     const u64 stream = apr ? r.nnz * ((u64)r.nmode * (8 + fsz) + 24) : 0;
-    return std::max(build_peak, resident + pi + stream) + model + (16ull << 20);
+    return std::max(build_peak, resident + kept + pi + stream) + model + (16ull << 20);
 }
 
 struct Job {

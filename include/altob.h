@@ -75,7 +75,8 @@ typedef struct {
     uint64_t cr_masks[ALTOB_MAX_MODES][2];
     uint64_t alto_mask[2];
     uint64_t alto_cr_mask[2];
-    uint64_t device_bytes; /* HBM held by the handle */
+    uint64_t device_bytes; /* HBM held by the handle, with the buffers it keeps between calls;
+                              the tile plans are in plan_bytes */
     uint64_t key_bytes;    /* bytes of index stored per nonzero on the device */
     int nruns;             /* high index words kept as a run table (0: none) */
     int plan_modes;        /* bit n set: mode n has a tile plan (MTTKRP) */
@@ -104,7 +105,8 @@ ALTOB_API const char* altob_version(void);
  * device's memory between calls instead of handing it back to the system at
  * every synchronisation; this returns what is unused on the current device
  * (the driver also takes it back when another allocation of the process needs
- * it).  Memory still in use by work in flight is not waited for. */
+ * it).  Memory still in use by work in flight is not waited for, and what a
+ * handle keeps between calls (altob_info) stays with it until altob_destroy. */
 ALTOB_API altob_status altob_trim_memory(void);
 
 /* ---- tensor build ------------------------------------------------------
