@@ -312,7 +312,8 @@ static altob_status run_padded(altob_tensor* t, int mode, void* const* dU, void*
     pa.Rp = (int)Rp;
     k_pad_rows<FT><<<dim3(pad_grid(most, (int)Rp), n), 256, 0, st>>>(pa);
     ALTOB_LAUNCH_CHECK();
-    ALTOB_TRY((run_tiled_vt<FT, VT>(t, mode, pU, po, Rp, phi, eps, perm, true, flags & MT_RUN_SUMS, st)));
+    ALTOB_TRY((run_tiled_vt<FT, VT>(t, mode, pU, po, Rp, phi, eps, perm, true, (flags & MT_RUN_SUMS) | MT_PADDED,
+                                       st)));
     k_unpad_add<FT><<<pad_grid(t->dims[mode], (int)R), 256, 0, st>>>((FT*)dout, po, t->dims[mode], (int)R, (int)Rp);
     ALTOB_LAUNCH_CHECK();
     *ran = true;
@@ -443,8 +444,13 @@ static altob_status run_tiled_vt(altob_tensor* t, int mode, void* const* dU, voi
         // and graphs of one handle may be replayed side by side.
         const bool apart = sizeof(FT) == 8 && stream_capturing(st);
         if (apart || (sizeof(FT) == 8 && per_cta < 4)) a.hot = 0;
-        // through oidx a long run is a row's whole range: the grouped kernel's line
-        if (perm && sizeof(FT) == 4) a.hot_minrun = GT_HOT_MINRUN;
+        // the grouped kernel's line of 8 for the FP32 calls that it used to run,
+        // whose error would grow with 16 (Phi of three modes of 18.9M counts at
+        // rank 16: 2.93, 4.59 and 6.86e-7 from FP64 at 8, 3.09, 4.79 and 7.11e-7
+        // at 16; 1.89 against 1.86 ms for all four modes), and for shared tiles,
+        // whose shorter stretches cut the long runs (150,001 nonzeros of order
+        // 5, 151 rows: 1.76e-7 at 8, 1.88e-7 at 16, the same time)
+        if (sizeof(FT) == 4 && (perm || phi || (flags & MT_PADDED) || a.split_shift)) a.hot_minrun = GT_HOT_MINRUN;
         // an output of at most WHOLE_BYTES is kept whole by every CTA that
         // takes enough tiles to repay clearing the copy and adding it up
         if (!apart && !perm && !(flags & MT_RUN_SUMS) && t->dims[mode] * R * sizeof(FT) <= WHOLE_BYTES &&

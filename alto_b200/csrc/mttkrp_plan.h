@@ -20,8 +20,8 @@ const uint16_t* tensor_plan(altob_tensor* t, int mode, cudaStream_t st);
 // flags: MT_AFTER_CLEAR: the last launch on st is finish_cols, which the MTTKRP
 // may overlap up to its first read of a factor; MT_RUN_SUMS: every run is
 // added to the output itself, also where the output is short (no per-CTA
-// copies).
-enum { MT_AFTER_CLEAR = 1, MT_RUN_SUMS = 2 };
+// copies); MT_PADDED: the factors are padded copies (set inside).
+enum { MT_AFTER_CLEAR = 1, MT_RUN_SUMS = 2, MT_PADDED = 4 };
 altob_status mttkrp_device(altob_tensor* t, int mode, altob_dtype ft, void* const* dU, u64 R, int accumulate,
                            altob_algo algo, cudaStream_t st, int flags = 0);
 altob_status phi_device(altob_tensor* t, int mode, altob_dtype ft, void* const* dU, u64 R, double eps,
