@@ -587,8 +587,10 @@ static altob_status cp_apr_impl(altob_tensor* t, FT** U, FT* lam_io, int R, int 
         std::vector<void*> tmpU(N);
         for (int n = 0; n < N; ++n) tmpU[n] = U[n];
         tmpU[N - 1] = mt;
-        // summed run by run: per-CTA copies of a short last mode would move the
-        // reported FP32 fit by about 1.5e-6 of its value
+        // summed run by run, as this fit always was: per-CTA copies of a short
+        // last mode would move the reported FP32 fit by about 1.5e-6 of its
+        // value (4.7M counts, fit 4.6e-7: 1.7e-6 from the FP64 solve's fit so,
+        // under 1e-7 with copies), away from what earlier runs reported
         ALTOB_TRY(mttkrp_device(t, N - 1, ft, tmpU.data(), (u64)R, 0, ALTOB_ALGO_AUTO, st, MT_RUN_SUMS));
     }
     ALTOB_TRY(gram<FT>(U[N - 1], t->dims[N - 1], R, s.G + (size_t)(N - 1) * R * R, nullptr, nullptr, mt, s.inner,
