@@ -440,10 +440,7 @@ static altob_status run_tiled_vt(altob_tensor* t, int mode, void* const* dU, voi
         // 2e-6 from FP64 without, 2.5e-7 with).  FP64 needs it for the contended
         // atomics only, and it repays clearing and adding it up from about four
         // tiles per CTA on.
-        // FP64 captures run without accumulators: they belong to the handle,
-        // and graphs of one handle may be replayed side by side.
-        const bool apart = sizeof(FT) == 8 && stream_capturing(st);
-        if (apart || (sizeof(FT) == 8 && per_cta < 4)) a.hot = 0;
+        if (sizeof(FT) == 8 && per_cta < 4) a.hot = 0;
         // the grouped kernel's line of 8 for the FP32 calls that it used to run,
         // whose error would grow with 16 (Phi of three modes of 18.9M counts at
         // rank 16: 2.93, 4.59 and 6.86e-7 from FP64 at 8, 3.09, 4.79 and 7.11e-7
@@ -453,11 +450,14 @@ static altob_status run_tiled_vt(altob_tensor* t, int mode, void* const* dU, voi
         if (sizeof(FT) == 4 && (perm || phi || (flags & MT_PADDED) || a.split_shift)) a.hot_minrun = GT_HOT_MINRUN;
         // an output of at most WHOLE_BYTES is kept whole by every CTA that
         // takes enough tiles to repay clearing the copy and adding it up
-        if (!apart && !perm && !(flags & MT_RUN_SUMS) && t->dims[mode] * R * sizeof(FT) <= WHOLE_BYTES &&
+        if (!perm && !(flags & MT_RUN_SUMS) && t->dims[mode] * R * sizeof(FT) <= WHOLE_BYTES &&
             t->dims[mode] <= 128 * per_cta && per_cta >= 2 && env_int("ALTOB_HOT_ROWS", 1)) {
             a.hot = 0;
             a.whole = (int)t->dims[mode];
         }
+        // FP64 captures run without accumulators: they belong to the handle,
+        // and graphs of one handle may be replayed side by side
+        if (sizeof(FT) == 8 && (a.hot || a.whole) && stream_capturing(st)) a.hot = a.whole = 0;
         ALTOB_TRY(set_hot_acc(t, a, c.grid.x, st));
         return launch_planned<FT, VT>(a, c, st, nullptr);
     }
